@@ -79,6 +79,20 @@ __device__ __forceinline__ void quat_apply_rotvec(float* q, float rx, float ry, 
     q[0] = w * nn; q[1] = x * nn; q[2] = y * nn; q[3] = z * nn;
 }
 
+// exp(x) = 2^(x log2 e) and 1 / sqrt(x) as the single hardware instructions that flush denormals. The compiler's
+// __expf and rsqrtf add a rescaling for denormal operands or results (3-4 instructions each); a term below 1e-38 adds
+// nothing to energies of kcal/mol size, and the distances are clamped far above it.
+__device__ __forceinline__ float exp_ftz(float x) {
+    float y;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(__fmul_rn(x, 1.44269504f)));
+    return y;
+}
+__device__ __forceinline__ float rsqrt_ftz(float x) {
+    float y;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+
 // Vina-family pair energy and dE/dr with the radius sum and the hydrophobic / H-bond pair flags precomputed.
 // Same terms as mckernel.py:44-64 / scoring.pair_terms . weights.
 struct PairPrm {
@@ -102,17 +116,17 @@ __host__ inline PairPrm make_pair_prm(const float* prm) {
 // to 0 (d >= bad); written as clamps and selects, which add exactly 0 where the piecewise form adds nothing.
 __device__ __forceinline__ float pair_energy(float r, float rsum, int flags, const PairPrm& p, float& de) {
     const float d = r - rsum;
-    const float u1 = (d - p.g1_off) * p.g1_inv, g1 = __expf(-u1 * u1);
-    const float u2 = (d - p.g2_off) * p.g2_inv, g2 = __expf(-u2 * u2);
+    const float u1 = (d - p.g1_off) * p.g1_inv, g1 = exp_ftz(-u1 * u1);
+    const float u2 = (d - p.g2_off) * p.g2_inv, g2 = exp_ftz(-u2 * u2);
     float e = p.w_g1 * g1 + p.w_g2 * g2;
     de = p.w_g1 * (-2.f * u1 * p.g1_inv) * g1 + p.w_g2 * (-2.f * u2 * p.g2_inv) * g2;
     const float dr = fminf(d - p.rep_off, 0.f);
     e += p.w_rep * dr * dr;
     de += p.w_rep * 2.f * dr;
     const float wh = (flags & PF_HYD) ? p.w_hyd : 0.f, wb = (flags & PF_HB) ? p.w_hb : 0.f;
-    const float vh = (p.hyd_bad - d) * p.hyd_inv, vb = (p.hb_bad - d) * p.hb_inv;
-    e += wh * fminf(fmaxf(vh, 0.f), 1.f);
-    e += wb * fminf(fmaxf(vb, 0.f), 1.f);
+    const float vh = __saturatef((p.hyd_bad - d) * p.hyd_inv), vb = __saturatef((p.hb_bad - d) * p.hb_inv);
+    e += wh * vh;
+    e += wb * vb;
     de -= (vh > 0.f && vh < 1.f) ? wh * p.hyd_inv : 0.f;
     de -= (vb > 0.f && vb < 1.f) ? wb * p.hb_inv : 0.f;
     return e;

@@ -68,12 +68,13 @@ __device__ int block_exclusive_scan(int flag, int* warp_tot, int* total) {
 }
 
 // ------------------------------------------------------------------------------------------ conformers
-// Ligand-frame heavy-atom coordinates of torsion set `trial` of ligand l into X ([3][AM] in shared memory) and
+// Ligand-frame heavy-atom coordinates of torsion set `trial` of ligand l (radii rad [AM]) into X ([3][AM] in shared
+// memory) and
 // the set's torsion angles into th (shared, KM); returns the intra-ligand energy (all lanes). Set 0 is the input
 // conformer (all angles 0); the others draw each torsion angle uniformly in [-pi, pi) from the counter-based
 // stream (seed, ligand, set, torsion).
-__device__ float conformer_set(const SearchParams& P, int l, int trial, unsigned long long seed, float* X, float* th,
-                               float* cs, float* sn, int lane) {
+__device__ float conformer_set(const SearchParams& P, int l, int trial, unsigned long long seed, const float* rad,
+                               float* X, float* th, float* cs, float* sn, int lane) {
     const int4 inf = P.info[l];
     const int na = inf.x, nt = inf.y, np = inf.z;
     const int AM = P.AM;
@@ -120,7 +121,7 @@ __device__ float conformer_set(const SearchParams& P, int l, int trial, unsigned
         const float r = sqrtf(rx * rx + ry * ry + rz * rz);
         if (r >= P.pp.cutoff) continue;
         float de;
-        e += pair_energy(r, __int_as_float(rec.y), fl, P.pp, de);
+        e += pair_energy(r, rad[i] + rad[j], fl, P.pp, de);
     }
     e = warp_sum(e);
     __syncwarp();
@@ -132,20 +133,26 @@ __device__ float conformer_set(const SearchParams& P, int l, int trial, unsigned
 // energies e [L, C].
 __global__ void __launch_bounds__(256) conformer_kernel(const __grid_constant__ SearchParams P, int NT, int C,
                                                         unsigned long long seed, float* theta_out, float* conf_out,
-                                                        float* e_out) {
+                                                        float* e_out, const __grid_constant__ TypeTables tt) {
     extern __shared__ float csm[];
     const int l = blockIdx.x;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
     const int AM = P.AM, KM = P.KM;
     float* e_s = csm;                           // [NT]
     int* sel = (int*)(csm + NT);                // [C]
-    float* ws = csm + NT + C + wid * (3 * AM + 3 * KM);
+    float* rad = csm + NT + C;                  // [AM]
+    float* ws = rad + AM + wid * (3 * AM + 3 * KM);
     float* X = ws;
     float* th = ws + 3 * AM;
     float* cs = th + KM;
     float* sn = cs + KM;
+    for (int a = threadIdx.x; a < AM; a += blockDim.x) {
+        const int typ = __float_as_int(P.atoms[(long long)l * AM + a].w) >> 16;
+        rad[a] = tt.radius[typ < 0 ? 0 : typ & 63];
+    }
+    __syncthreads();
     for (int t = wid; t < NT; t += nw) {
-        const float e = conformer_set(P, l, t, seed, X, th, cs, sn, lane);
+        const float e = conformer_set(P, l, t, seed, rad, X, th, cs, sn, lane);
         if (lane == 0) e_s[t] = (e == e) ? e : 3.4e38f;   // a NaN energy ranks last
     }
     __syncthreads();
@@ -161,7 +168,7 @@ __global__ void __launch_bounds__(256) conformer_kernel(const __grid_constant__ 
     __syncthreads();
     for (int r = wid; r < C; r += nw) {
         const int t = sel[r];
-        conformer_set(P, l, t, seed, X, th, cs, sn, lane);
+        conformer_set(P, l, t, seed, rad, X, th, cs, sn, lane);
         const long long o = (long long)l * C + r;
         for (int k = lane; k < KM; k += 32) theta_out[o * KM + k] = th[k];
         for (int a = lane; a < AM; a += 32) {
@@ -419,10 +426,10 @@ extern "C" int adock_conformers(const adock_ligands_t* lig, const adock_work_t* 
     ADOCK_CHECK_ARG(C >= 1 && C <= NT, "C must be in [1, NT] (got %d)", C);
     ADOCK_CHECK_ARG(theta && conf && e, "null array argument");
     const int threads = 256;
-    const size_t smem = ((size_t)NT + C + (threads / 32) * (3 * (size_t)P.AM + 3 * (size_t)P.KM)) * sizeof(float);
+    const size_t smem = ((size_t)NT + C + P.AM + (threads / 32) * (3 * (size_t)P.AM + 3 * (size_t)P.KM)) * sizeof(float);
     ADOCK_CUDA(cudaFuncSetAttribute(conformer_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     conformer_kernel<<<lig->L, threads, smem, (cudaStream_t)stream>>>(P, NT, C, splitmix(seed ^ 0xC0F0A11CE5ULL), theta,
-                                                                      conf, e);
+                                                                      conf, e, make_tables(sf));
     ADOCK_CUDA(cudaGetLastError());
     return ADOCK_OK;
 }

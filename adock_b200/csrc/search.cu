@@ -44,13 +44,13 @@ __global__ void prepare_kernel(adock_ligands_t lig, TypeTables tt, float4* atoms
 }
 
 // Intra-pair schedule (one warp per ligand): the np pairs are placed into R = ceil(np / 32) rounds of 32 slots.
-// eval_eg adds a pair's force to its first atom with one set of shared-memory atomics and to its second atom with
-// another, so within a round only repeats of an atom on the same side collide (and serialise the atomic). The
+// Forces are added per round and side, once more for every repeat of an atom on the same side of a round
+// (push_forces), so within a round only repeats of an atom on the same side cost time. The
 // Vina pair term is symmetric, so each pair may also be stored either way round. Greedy in pair order: over the
 // rounds with a free slot and both orientations, the choice where the larger of (the first atom's count as a first
 // atom, the second atom's count as a second atom) is smallest, then their sum, then the lowest round, then the
 // given orientation. Empty slots get x = -1. Counts live in dynamic shared memory, [R_cap][AM] per side; ligands
-// with more than R_cap rounds keep the pair order.
+// with more than R_cap rounds keep the pair order. The rounds' links are written last.
 __global__ void schedule_pairs_kernel(adock_ligands_t lig, TypeTables tt, int2* pairs, int P_pad, int R_cap) {
     extern __shared__ int sched_smem[];
     const int l = blockIdx.x, lane = threadIdx.x;
@@ -67,10 +67,31 @@ __global__ void schedule_pairs_kernel(adock_ligands_t lig, TypeTables tt, int2* 
         tj = tj < 0 ? 0 : (tj & 63);
         const int fl = hyd_pair(tt.flags[ti], tt.flags[tj]) | hb_pair(tt.flags[ti], tt.flags[tj]);
         const int a = swap ? j : i, b = swap ? i : j;
-        return make_int2((a & 0xff) | ((b & 0xff) << 8) | (fl << 16), __float_as_int(tt.radius[ti] + tt.radius[tj]));
+        return make_int2((a & 0xff) | ((b & 0xff) << 8) | (fl << 16), 0);
+    };
+    // How the slots of each written round share atoms (see PR_NEXT).
+    auto link_rounds = [&]() {
+        for (int r = 0; r < R; ++r) {
+            int2 v = out[r * 32 + lane];
+            int links = 0;
+            v.y = 0;
+#pragma unroll
+            for (int side = 0; side < 2; ++side) {
+                const int a = v.x < 0 ? 256 + lane : (v.x >> (8 * side)) & 0xff;   // an empty slot matches no other
+                const unsigned same = __match_any_sync(0xffffffffu, a);
+                const unsigned above = lane == 31 ? 0u : same & (0xffffffffu << (lane + 1));
+                links |= (above ? __ffs(above) - 1 : lane) << (PR_NEXT + 5 * side);
+                links |= ((same & ((1u << lane) - 1u)) ? 0 : 1) << (PR_LEAD + side);
+                v.y |= (__reduce_max_sync(0xffffffffu, __popc(same)) - 1) << (5 * side);
+            }
+            if (v.x >= 0) v.x |= links;
+            out[r * 32 + lane] = v;
+        }
     };
     if (R > R_cap) {  // very large ligands: keep the pair order
         for (int q = lane; q < P_pad; q += 32) out[q] = q < np ? record(q, 0) : make_int2(-1, 0);
+        __syncwarp();
+        link_rounds();
         return;
     }
     for (int r = lane; r < R; r += 32) {
@@ -109,6 +130,8 @@ __global__ void schedule_pairs_kernel(adock_ligands_t lig, TypeTables tt, int2* 
         const int r = q >> 5;
         if (r >= R || (q & 31) >= fill[r]) out[q] = make_int2(-1, 0);
     }
+    __syncwarp();
+    link_rounds();
 }
 
 // ------------------------------------------------------------------------------------------ pose coordinates

@@ -14,24 +14,26 @@ namespace adock {
 #define EPSF 1.1920929e-07f
 
 // Code-size knobs of the MC kernel (instruction-cache footprint vs register allocation across calls).
-#ifdef ADOCK_BFGS_INLINE
-#define ADOCK_BFGS_ATTR __forceinline__
-#else
-#define ADOCK_BFGS_ATTR __noinline__
-#endif
 #ifdef ADOCK_COLD_NOINLINE
 #define ADOCK_COLD_ATTR __noinline__
 #else
 #define ADOCK_COLD_ATTR __forceinline__
 #endif
 #define PAIR_ROUNDS_MAX 256   // pair schedule: at most 256 rounds of 32 (8,192 pairs) are reordered
+// Intra-pair records: a ligand's pairs are scheduled in rounds of 32 slots, one per lane. x: first atom (bits 0-7),
+// second atom (8-15), flags (16-17), and how the slots of a round share atoms: the next higher lane with the same first
+// atom (18-22; the lane itself if none) and with the same second atom (23-27), and whether the slot is the first with
+// its first atom (28) and with its second atom (29). Empty slots are -1. y: how many more slots the round's most
+// repeated first atom (bits 0-4) and second atom (5-9) have.
+#define PR_NEXT 18    // + 5 * side
+#define PR_LEAD 28    // + side
 
 struct SearchParams {
     // B200 working layout
     const float4* atoms;   // [L, AM]
     const uint32_t* masks; // [L, AM]
     const float4* tors;    // [L, KM, 2]
-    const int2* pairs;     // [L, P_pad] scheduled in rounds of 32; empty slots have x = -1
+    const int2* pairs;     // [L, P_pad] records (PR_NEXT), scheduled in rounds of 32
     const int4* info;      // [L] na, nt, np, rec_idx
     const float* rg;       // [L]
     int AM, KM, P, P_pad;
@@ -114,17 +116,17 @@ __device__ __forceinline__ void stage_tables(TypeTables& dst, const TypeTables& 
 // ------------------------------------------------------------------------------------------ per-warp workspace
 // Float offsets of the per-warp shared workspace for a given AM / KM (float4 arrays first).
 struct WSLayout {
-    int X, FF, ap, au, tp, tu, mk, ax, cs, sn, H, x, xn, xo, cur, best, g, gn, go, p, y, mhy, total;
+    int X, FT, ap, au, tp, tu, ax, cs, sn, H, x, xn, xo, cur, best, g, gn, go, p, y, mhy, total;
     __host__ __device__ WSLayout(int AM, int KM) {
         const int DM = 6 + KM, SD = 7 + KM;
         int o = 0;
-        X = o; o += 3 * AM;    // world coordinates, [3][AM] (x, y, z arrays)
-        FF = o; o += 3 * AM;   // forces, [3][AM]
+        X = o; o += 4 * AM;    // world coordinates and radii, [4][AM] (x, y, z, radius arrays)
+        FT = o; o += 8 * AM;   // forces of the pair loop, [3][AM]; then float4 (force, torsion bitmask) and float4
+                               // (torque, 0) per atom
         ap = o; o += 4 * KM;
         au = o; o += 4 * KM;
         tp = o; o += 4 * KM;
         tu = o; o += 4 * KM;
-        mk = o; o += AM;
         ax = o; o += KM;      // packed axis atom indices (a0 | a1 << 16)
         cs = o; o += KM;
         sn = o; o += KM;
@@ -167,8 +169,8 @@ struct Chain {
 };
 
 template <int APL, typename GT>
-__device__ __forceinline__ void load_chain(Chain<APL>& c, const SearchParams& P, int l, float* ws, const WSLayout& L,
-                                           int lane, int exact, const int* nb, int nbn) {
+__device__ __forceinline__ void load_chain(Chain<APL>& c, const SearchParams& P, const TypeTables& tt, int l, float* ws,
+                                           const WSLayout& L, int lane, int exact, const int* nb, int nbn) {
     const int4 inf = P.info[l];
     c.na = inf.x; c.nt = inf.y; c.np = inf.z;
     c.nrounds = (inf.z + 31) >> 5;
@@ -190,7 +192,6 @@ __device__ __forceinline__ void load_chain(Chain<APL>& c, const SearchParams& P,
     c.nb = nb; c.nbn = nbn;
     const float4* at = P.atoms + (long long)l * P.AM;
     const uint32_t* mk = P.masks + (long long)l * P.AM;
-    uint32_t* smk = (uint32_t*)(ws + L.mk);
 #pragma unroll
     for (int i = 0; i < APL; ++i) {
         const int a = lane + 32 * i;
@@ -200,7 +201,7 @@ __device__ __forceinline__ void load_chain(Chain<APL>& c, const SearchParams& P,
         c.slot[i] = meta & 0xffff;
         c.typ[i] = meta >> 16;
         c.mask[i] = mk[a];
-        smk[a] = c.mask[i];
+        ws[L.X + 3 * 32 * APL + a] = tt.radius[c.typ[i] < 0 ? 0 : c.typ[i] & 63];
     }
     const float4* tr = P.tors + (long long)l * P.KM * 2;
     float4* ap = (float4*)(ws + L.ap);
@@ -249,24 +250,109 @@ __device__ __forceinline__ float trilinear(const GT* G, int ny, int nz, const fl
     return e;
 }
 
-// Intra-ligand pair term of one scheduled slot: energy, and the force added into both atoms' entries. Positions X
-// and forces F are three arrays of AM floats each (x, y, z), so that 32 lanes touching 32 different atoms hit 32
-// different shared-memory banks (a float4 per atom would put the x components of 32 atoms on 8 banks).
+// Intra-ligand pair term of one scheduled slot: energy and the force on the first atom, 0 for an empty slot and beyond
+// the cutoff. Positions and radii are four arrays of AM floats, so that 32 lanes touching 32 different atoms hit 32
+// different shared-memory banks (a float4 per atom would put the x components of 32 atoms on 8 banks). Branch-free, so
+// that the slots a lane has in flight overlap.
 template <int AM>
-__device__ __forceinline__ float pair_slot(int2 pr, const float* X, float* F, const PairPrm& pp) {
-    if (pr.x < 0) return 0.f;
-    const int i = pr.x & 0xff, j = (pr.x >> 8) & 0xff, fl = pr.x >> 16;
-    const float rx = X[i] - X[j], ry = X[AM + i] - X[AM + j], rz = X[2 * AM + i] - X[2 * AM + j];
+__device__ __forceinline__ float pair_slot(int w, bool valid, const float* X, const PairPrm& pp, float3& f) {
+    const float *Xi = X + (w & 0xff), *Xj = X + ((w >> 8) & 0xff);
+    const float rx = Xi[0] - Xj[0], ry = Xi[AM] - Xj[AM], rz = Xi[2 * AM] - Xj[2 * AM];
     // r and 1/r from one reciprocal square root; clamping r^2 at 1e-12 is the reference's max(r, 1e-6)
     const float r2 = rx * rx + ry * ry + rz * rz;
-    const float rinv = rsqrtf(fmaxf(r2, 1e-12f));
+    const float rinv = rsqrt_ftz(fmaxf(r2, 1e-12f));
     const float r = r2 * rinv;
-    if (r >= pp.cutoff) return 0.f;
+    const bool on = valid && !(r >= pp.cutoff);
     float de;
-    const float e = pair_energy(r, __int_as_float(pr.y), fl, pp, de);
-    const float sc = de * rinv;
-    atomicAdd(F + i, sc * rx); atomicAdd(F + AM + i, sc * ry); atomicAdd(F + 2 * AM + i, sc * rz);
-    atomicAdd(F + j, -sc * rx); atomicAdd(F + AM + j, -sc * ry); atomicAdd(F + 2 * AM + j, -sc * rz);
+    const float e = pair_energy(r, Xi[3 * AM] + Xj[3 * AM], w >> 16, pp, de);
+    const float sc = on ? de * rinv : 0.f;
+    f.x = __fmul_rn(sc, rx); f.y = __fmul_rn(sc, ry); f.z = __fmul_rn(sc, rz);
+    return on ? e : 0.f;
+}
+
+// Adds one side of a round's pair forces to the forces F [3][AM]. Lanes that share an atom on the side form a chain in
+// lane order (see PR_NEXT); its first lane adds the members' forces, fetched by shuffles, and alone updates the entry.
+// Shared float atomics give the same sums (lanes that meet on an atom add in lane order) but serialise there.
+template <int AM, int SIDE>
+__device__ __forceinline__ void push_forces(int w, int repeats, float3 f, float* F) {
+    const int next = (w >> (PR_NEXT + 5 * SIDE)) & 31;
+    float* Fa = F + ((w >> (8 * SIDE)) & 0xff);
+    float sx, sy, sz;
+    if (SIDE) {
+        sx = __fsub_rn(Fa[0], f.x); sy = __fsub_rn(Fa[AM], f.y); sz = __fsub_rn(Fa[2 * AM], f.z);
+    } else {
+        sx = __fadd_rn(Fa[0], f.x); sy = __fadd_rn(Fa[AM], f.y); sz = __fadd_rn(Fa[2 * AM], f.z);
+    }
+    int src = next;
+    bool ok = src != (threadIdx.x & 31);
+#pragma unroll 1
+    for (int k = repeats; k > 0; --k) {
+        const float vx = __shfl_sync(0xffffffffu, f.x, src), vy = __shfl_sync(0xffffffffu, f.y, src),
+                    vz = __shfl_sync(0xffffffffu, f.z, src);
+        const int n = __shfl_sync(0xffffffffu, next, src);
+        if (ok) {
+            sx = SIDE ? __fsub_rn(sx, vx) : __fadd_rn(sx, vx);
+            sy = SIDE ? __fsub_rn(sy, vy) : __fadd_rn(sy, vy);
+            sz = SIDE ? __fsub_rn(sz, vz) : __fadd_rn(sz, vz);
+        }
+        ok = ok && n != src;
+        src = n;
+    }
+    if ((w >> (PR_LEAD + SIDE)) & 1) {
+        Fa[0] = sx;
+        Fa[AM] = sy;
+        Fa[2 * AM] = sz;
+    }
+    __syncwarp();
+}
+
+// Intra-ligand pairs: adds the lane's slots to its share e of the energy (returned) and the forces on the lane's atoms
+// (lane + 32 i) to F. An atom's contributions are added in the order round, first atoms before second atoms, lane.
+// Bound by instruction issue and the latency of the rounds' shared-memory updates (about 95 instructions per slot for
+// the pair term, 66 per round for the two sides). With shared float atomics for the forces and the pair parameters read
+// through a generic pointer this loop took 10.3 k of a single warp's 19 k cycles per evaluation (24 atoms, 7 rounds);
+// now 4.3 k. Summing in registers instead was slower: owners pulling by shuffles (132 instructions per round), or
+// per-atom slot lists over forces left in shared memory (12 wavefronts per entry from bank conflicts).
+template <int APL>
+__device__ __forceinline__ float pair_terms(float* ws, const WSLayout& L, const Chain<APL>& c, const PairPrm& pp,
+                                            float3 (&F)[APL], float e, int lane) {
+    constexpr int AM = 32 * APL;
+    const float* X = ws + L.X;
+    float* FF = ws + L.FT;
+#pragma unroll
+    for (int i = 0; i < APL; ++i) {
+        const int a = lane + 32 * i;
+        FF[a] = F[i].x; FF[AM + a] = F[i].y; FF[2 * AM + a] = F[i].z;
+    }
+    __syncwarp();
+    // two rounds in flight; the next two rounds' records are loaded while these are evaluated
+    const int empty = lane * (33 << PR_NEXT);   // atom 0 twice, linked to itself, first of nothing
+    const int2 none = make_int2(-1, 0);
+    int2 pa = c.nrounds > 0 ? c.pairs[lane] : none;
+    int2 pb = c.nrounds > 1 ? c.pairs[32 + lane] : none;
+#pragma unroll 1
+    for (int r = 0; r < c.nrounds; r += 2) {
+        const int2 qa = (r + 2 < c.nrounds) ? c.pairs[(r + 2) * 32 + lane] : none;
+        const int2 qb = (r + 3 < c.nrounds) ? c.pairs[(r + 3) * 32 + lane] : none;
+        const int wa = pa.x < 0 ? empty : pa.x, wb = pb.x < 0 ? empty : pb.x;
+        float3 fa, fb;
+        e += pair_slot<AM>(wa, pa.x >= 0, X, pp, fa);
+        e += pair_slot<AM>(wb, pb.x >= 0, X, pp, fb);
+        push_forces<AM, 0>(wa, pa.y & 31, fa, FF);
+        push_forces<AM, 1>(wa, pa.y >> 5, fa, FF);
+        if (r + 1 < c.nrounds) {
+            push_forces<AM, 0>(wb, pb.y & 31, fb, FF);
+            push_forces<AM, 1>(wb, pb.y >> 5, fb, FF);
+        }
+        pa = qa;
+        pb = qb;
+    }
+#pragma unroll
+    for (int i = 0; i < APL; ++i) {
+        const int a = lane + 32 * i;
+        F[i] = make_float3(FF[a], FF[AM + a], FF[2 * AM + a]);
+    }
+    __syncwarp();
     return e;
 }
 
@@ -281,13 +367,11 @@ template <int APL, typename GT, bool EX>
 __device__ __forceinline__ float eval_eg(float* ws, const WSLayout& L, const float* s, float* g, const Chain<APL>& c,
                          const SearchParams& P, const TypeTables& tt, int lane) {
     constexpr int AM = 32 * APL;
-    float* X = ws + L.X;     // [3][AM] world coordinates
-    float* FF = ws + L.FF;   // [3][AM] forces dE/dX
+    float* X = ws + L.X;     // [3][AM] world coordinates (radii behind them)
     const float4* ap = (const float4*)(ws + L.ap);
     const float4* au = (const float4*)(ws + L.au);
     float4* tp = (float4*)(ws + L.tp);
     float4* tu = (float4*)(ws + L.tu);
-    const uint32_t* smk = (const uint32_t*)(ws + L.mk);
     const int* axs = (const int*)(ws + L.ax);
     float* cs = ws + L.cs;
     float* sn = ws + L.sn;
@@ -307,10 +391,12 @@ __device__ __forceinline__ float eval_eg(float* ws, const WSLayout& L, const flo
     }
     __syncwarp();
     float e = 0.f;
+    float3 F[APL];   // dE/dX of the lane's atoms
     const GT* grid = (const GT*)c.grid;
 #pragma unroll
     for (int i = 0; i < APL; ++i) {
         const int a = lane + 32 * i;
+        F[i] = make_float3(0.f, 0.f, 0.f);
         if (a < c.na) {
             float px = c.ref[i].x, py = c.ref[i].y, pz = c.ref[i].z;
             uint32_t m = c.mask[i];
@@ -367,28 +453,11 @@ __device__ __forceinline__ float eval_eg(float* ws, const WSLayout& L, const flo
                 gg[d] += P.pen * (-2.f * lo + 2.f * hi);
             }
             e += ea;
-            FF[a] = gg[0];
-            FF[AM + a] = gg[1];
-            FF[2 * AM + a] = gg[2];
+            F[i] = make_float3(gg[0], gg[1], gg[2]);
         }
     }
     __syncwarp();
-    // intra-ligand pairs, scheduled in rounds of 32 in which an atom appears at most once (adock_prepare), so the
-    // force atomics of one round do not collide; two rounds in flight per iteration
-    // the next two rounds' records are loaded while the current two are evaluated
-    {
-        const int2 none = make_int2(-1, 0);
-        int2 pa = c.nrounds > 0 ? c.pairs[lane] : none;
-        int2 pb = c.nrounds > 1 ? c.pairs[32 + lane] : none;
-        for (int r = 0; r < c.nrounds; r += 2) {
-            const int2 qa = (r + 2 < c.nrounds) ? c.pairs[(r + 2) * 32 + lane] : none;
-            const int2 qb = (r + 3 < c.nrounds) ? c.pairs[(r + 3) * 32 + lane] : none;
-            e += pair_slot<AM>(pa, X, FF, P.pp);
-            e += pair_slot<AM>(pb, X, FF, P.pp);
-            pa = qa;
-            pb = qb;
-        }
-    }
+    e = pair_terms<APL>(ws, L, c, P.pp, F, e, lane);
     // world torsion axes (axis atoms' current positions)
     for (int k = lane; k < c.nt; k += 32) {
         const int a0 = axs[k] & 0xffff, a1 = axs[k] >> 16;
@@ -398,6 +467,19 @@ __device__ __forceinline__ float eval_eg(float* ws, const WSLayout& L, const flo
         tp[k] = make_float4(Ax - t0, Ay - t1, Az - t2, 0.f);
         tu[k] = make_float4(ux * nn, uy * nn, uz * nn, 0.f);
     }
+    // each atom's force with its torsion bitmask, and its torque (X - t) x F
+    float4* FA = (float4*)(ws + L.FT);
+    float4* TA = FA + AM;
+#pragma unroll
+    for (int i = 0; i < APL; ++i) {
+        const int a = lane + 32 * i;
+        if (a < c.na) {
+            const float Fx = F[i].x, Fy = F[i].y, Fz = F[i].z;
+            const float dx = X[a] - t0, dy = X[AM + a] - t1, dz = X[2 * AM + a] - t2;
+            FA[a] = make_float4(Fx, Fy, Fz, __uint_as_float(c.mask[i]));
+            TA[a] = make_float4(dy * Fz - dz * Fy, dz * Fx - dx * Fz, dx * Fy - dy * Fx, 0.f);
+        }
+    }
     __syncwarp();
     // subtree sums of F and (X - t) x F: sum k < nt is torsion k's subtree, sum k == nt is the whole ligand.
     // The nt + 1 sums are spread over all 32 lanes: G lanes per atom chunk (G = next power of two >= nt + 1),
@@ -406,16 +488,14 @@ __device__ __forceinline__ float eval_eg(float* ws, const WSLayout& L, const flo
         const int G = c.nt < 1 ? 1 : (c.nt < 3 ? 4 : (c.nt < 7 ? 8 : (c.nt < 15 ? 16 : 32)));
         const int k = lane & (G - 1), chunk = lane / G, C = 32 / G;
         float S0 = 0.f, S1 = 0.f, S2 = 0.f, T0 = 0.f, T1 = 0.f, T2 = 0.f;
-        if (k <= c.nt) {
-            const uint32_t bit = (k == c.nt) ? 0xffffffffu : (1u << k);
-            const bool all = (k == c.nt);
-            for (int a = chunk; a < c.na; a += C) {
-                if (all || (smk[a] & bit)) {
-                    const float Fx = FF[a], Fy = FF[AM + a], Fz = FF[2 * AM + a];
-                    const float dx = X[a] - t0, dy = X[AM + a] - t1, dz = X[2 * AM + a] - t2;
-                    S0 += Fx; S1 += Fy; S2 += Fz;
-                    T0 += dy * Fz - dz * Fy; T1 += dz * Fx - dx * Fz; T2 += dx * Fy - dy * Fx;
-                }
+        const uint32_t bit = k < c.nt ? 1u << k : 0u;
+        const bool all = k == c.nt;
+#pragma unroll 4
+        for (int a = chunk; a < c.na; a += C) {
+            const float4 f = FA[a], t = TA[a];
+            if (all || (__float_as_uint(f.w) & bit)) {
+                S0 += f.x; S1 += f.y; S2 += f.z;
+                T0 += t.x; T1 += t.y; T2 += t.z;
             }
         }
         for (int o = G; o < 32; o <<= 1) {
@@ -440,11 +520,10 @@ __device__ __forceinline__ float eval_eg(float* ws, const WSLayout& L, const flo
             const bool all = (k == c.nt);
             const uint32_t bit = all ? 0u : (1u << k);
             for (int a = 0; a < c.na; ++a) {
-                if (all || (smk[a] & bit)) {
-                    const float Fx = FF[a], Fy = FF[AM + a], Fz = FF[2 * AM + a];
-                    const float dx = X[a] - t0, dy = X[AM + a] - t1, dz = X[2 * AM + a] - t2;
-                    S0 += Fx; S1 += Fy; S2 += Fz;
-                    T0 += dy * Fz - dz * Fy; T1 += dz * Fx - dx * Fz; T2 += dx * Fy - dy * Fx;
+                const float4 f = FA[a], t = TA[a];
+                if (all || (__float_as_uint(f.w) & bit)) {
+                    S0 += f.x; S1 += f.y; S2 += f.z;
+                    T0 += t.x; T1 += t.y; T2 += t.z;
                 }
             }
             if (all) {
@@ -502,13 +581,12 @@ __device__ __forceinline__ void neg_hv(const float* H, const float* v, float* ou
 
 // Vina-1.2-style BFGS on state x (shared, in/out); returns the final energy (mckernel.py:267-326).
 // The curvature scalar y.p and the update guard alpha * y.p >= eps are evaluated in float64.
-// Not inlined: the MC kernel calls it from two sites (start optimisation and every step); one copy, with one
-// inlined eval_eg, keeps the kernel small enough for the instruction cache (instruction-fetch stalls were the
-// largest stall reason with four inlined copies of eval_eg).
+// Inlined at the MC kernel's one call site, with one inlined eval_eg: one copy keeps the kernel small enough for the
+// instruction cache, and the pair parameters stay constant-bank operands. (As a function of its own it read them
+// through a generic pointer, again after every shared-memory store of the pair loop.)
 template <int APL, typename GT, bool EX>
-__device__ ADOCK_BFGS_ATTR float bfgs(float* ws, const WSLayout& L, float* x, int iters, const Chain<APL>& c_in,
-                                   const SearchParams& P, const TypeTables& tt, int lane, unsigned& n_eval) {
-    const Chain<APL> c = c_in;   // registers for the whole optimisation
+__device__ __forceinline__ float bfgs(float* ws, const WSLayout& L, float* x, int iters, const Chain<APL>& c,
+                                      const SearchParams& P, const TypeTables& tt, int lane, unsigned& n_eval) {
     const int D = 6 + c.nt, S = 7 + c.nt;
     float* H = ws + L.H;
     float* g = ws + L.g;
@@ -748,7 +826,7 @@ __global__ void __launch_bounds__(128, MINB) mc_kernel(const __grid_constant__ S
         Chain<APL> c;
         const int* nb = M.nbr ? M.nbr + (long long)ch * M.nb_max : nullptr;
         const int nbn = M.nbr ? M.nbr_n[ch] : 0;
-        load_chain<APL, GT>(c, P, l, ws, L, lane, M.exact, nb, nbn);
+        load_chain<APL, GT>(c, P, tt, l, ws, L, lane, M.exact, nb, nbn);
         const int S = 7 + c.nt;
         const int iters = M.bfgs_iters > 0 ? M.bfgs_iters : (25 + c.na) / 3;
         float* cur = ws + L.cur;
@@ -761,67 +839,70 @@ __global__ void __launch_bounds__(128, MINB) mc_kernel(const __grid_constant__ S
             best[i] = gbest[i];
         }
         __syncwarp();
-        float ec, eb = M.best_e[ch];
-        if (M.init_opt) ec = bfgs<APL, GT, EX>(ws, L, cur, iters, c, P, tt, lane, n_eval);
-        else ec = M.cur_e[ch];
-        if (ec < eb) {
+        float ec = M.cur_e[ch], eb = M.best_e[ch];
+        int prop_fail = 0;
+        unsigned long long n_prop = 0, n_prop_acc = 0, n_plain = 0, n_plain_acc = 0;
+        if (!M.init_opt && ec < eb) {
             eb = ec;
             wcopy(best, cur, S, lane);
         }
-        int prop_fail = 0;
-        unsigned long long n_prop = 0, n_prop_acc = 0, n_plain = 0, n_plain_acc = 0;
-        for (int st = 0; st < M.mc_steps; ++st) {
+        // step -1 is the start optimisation: BFGS from the current state, taken without a test
+        for (int st = M.init_opt ? -1 : 0; st < M.mc_steps; ++st) {
+            const bool init = st < 0;
             const int sg = M.step_offset + st;
             wcopy(x, cur, S, lane);
             // learned move while the proposal has not failed PROP_FAIL_MAX times in a row, else plain MC
-            const bool use_prop = M.prop && prop_fail < PROP_FAIL_MAX &&
+            const bool use_prop = !init && M.prop && prop_fail < PROP_FAIL_MAX &&
                                   (M.prop_frac >= 1.f || uniform01(M.seed, cid, sg, 3) < M.prop_frac);
-            bool skip = false;   // a non-finite learned target: rejected without optimisation
-            if (use_prop) {
-                // the proposed target state (drawn around the state the network read at the segment start); with
-                // several tries per step, each candidate is evaluated once and the lowest-energy one is kept
-                const int T = M.prop_tries > 1 ? M.prop_tries : 1;
-                const float* mv0 = M.prop + ((long long)ch * M.prop_k + (long long)(st % (M.prop_k / T)) * T) * PROP_MOVE;
-                int pick = 0;
-                if (T > 1) {
-                    float e_min = 3.4e38f;
-                    for (int tr = 0; tr < T; ++tr) {
-                        const float* mv = mv0 + (long long)tr * PROP_MOVE;
-                        for (int i = lane; i < S; i += 32) x[i] = cur[i];
-                        __syncwarp();
-                        if (lane < 7) x[lane] = mv[lane];
-                        for (int k = lane; k < c.nt && k < 20; k += 32) x[7 + k] = mv[7 + k];
-                        __syncwarp();
-                        if (!target_finite(x, c.nt, lane)) continue;
-                        const float et = bfgs<APL, GT, EX>(ws, L, x, 0, c, P, tt, lane, n_eval);   // one evaluation
-                        if (et < e_min) { e_min = et; pick = tr; }
+            // The proposed target state (drawn around the state the network read at the segment start). With T > 1
+            // tries per step, passes 0..T-1 of the loop below evaluate one candidate each and the last pass
+            // optimises the lowest-energy one; all other steps take the last pass only.
+            const int T = use_prop && M.prop_tries > 1 ? M.prop_tries : 0;
+            const float* mv0 = use_prop ? M.prop + ((long long)ch * M.prop_k +
+                                                    (long long)(st % (M.prop_k / M.prop_tries)) * M.prop_tries) * PROP_MOVE
+                                        : nullptr;
+            int pick = 0;
+            float e_min = 3.4e38f, en = 3.4e38f;   // a non-finite learned target keeps en: rejected without optimisation
+            for (int tr = 0; tr <= T; ++tr) {
+                const bool last = tr == T;
+                if (use_prop) {
+                    if (tr > 0) wcopy(x, cur, S, lane);
+                    const float* mv = mv0 + (long long)(last ? pick : tr) * PROP_MOVE;
+                    if (lane < 7) x[lane] = mv[lane];
+                    for (int k = lane; k < c.nt && k < 20; k += 32) x[7 + k] = mv[7 + k];
+                    __syncwarp();
+                    if (!target_finite(x, c.nt, lane)) continue;
+                } else if (!init) {
+                    const int nm = 2 + c.nt;
+                    const int which = min((int)(uniform01(M.seed, cid, sg, 0) * nm), nm - 1);
+                    if (lane == 0) {
+                        float v[3];
+                        if (which == 0) {
+                            unit_ball(M.seed, cid, sg, 10, v);
+                            x[0] += M.amp_pos * v[0]; x[1] += M.amp_pos * v[1]; x[2] += M.amp_pos * v[2];
+                        } else if (which == 1) {
+                            unit_ball(M.seed, cid, sg, 10, v);
+                            const float sc = M.amp_rot / fmaxf(c.rg, 1.0f);
+                            quat_apply_rotvec(x + 3, sc * v[0], sc * v[1], sc * v[2]);
+                        } else {
+                            x[7 + which - 2] = (2.f * uniform01(M.seed, cid, sg, 1) - 1.f) * 3.14159265f;
+                        }
                     }
-                    wcopy(x, cur, S, lane);
+                    __syncwarp();
                 }
-                const float* mv = mv0 + (long long)pick * PROP_MOVE;
-                if (lane < 7) x[lane] = mv[lane];
-                for (int k = lane; k < c.nt && k < 20; k += 32) x[7 + k] = mv[7 + k];
-                __syncwarp();
-                skip = !target_finite(x, c.nt, lane);
-            } else {
-                const int nm = 2 + c.nt;
-                const int which = min((int)(uniform01(M.seed, cid, sg, 0) * nm), nm - 1);
-                if (lane == 0) {
-                    float v[3];
-                    if (which == 0) {
-                        unit_ball(M.seed, cid, sg, 10, v);
-                        x[0] += M.amp_pos * v[0]; x[1] += M.amp_pos * v[1]; x[2] += M.amp_pos * v[2];
-                    } else if (which == 1) {
-                        unit_ball(M.seed, cid, sg, 10, v);
-                        const float sc = M.amp_rot / fmaxf(c.rg, 1.0f);
-                        quat_apply_rotvec(x + 3, sc * v[0], sc * v[1], sc * v[2]);
-                    } else {
-                        x[7 + which - 2] = (2.f * uniform01(M.seed, cid, sg, 1) - 1.f) * 3.14159265f;
-                    }
-                }
+                const float et = bfgs<APL, GT, EX>(ws, L, x, last ? iters : 0, c, P, tt, lane, n_eval);
+                if (last) en = et;
+                else if (et < e_min) { e_min = et; pick = tr; }
             }
-            __syncwarp();
-            const float en = skip ? 3.4e38f : bfgs<APL, GT, EX>(ws, L, x, iters, c, P, tt, lane, n_eval);
+            if (init) {
+                ec = en;
+                wcopy(cur, x, S, lane);
+                if (ec < eb) {
+                    eb = ec;
+                    wcopy(best, x, S, lane);
+                }
+                continue;
+            }
             const bool accept =
                 isfinite(en) && ((en < ec) || (uniform01(M.seed, cid, sg, 2) < __expf((ec - en) / M.temp)));
             if (use_prop) { ++n_prop; n_prop_acc += accept; } else { ++n_plain; n_plain_acc += accept; }
@@ -882,7 +963,7 @@ __global__ void __launch_bounds__(128) eg_kernel(const __grid_constant__ SearchP
     for (int ch = blockIdx.x * (blockDim.x >> 5) + wid; ch < n; ch += warps) {
         const int l = chain_lig[ch];
         Chain<APL> c;
-        load_chain<APL, GT>(c, P, l, ws, L, lane, exact, nullptr, 0);
+        load_chain<APL, GT>(c, P, tt, l, ws, L, lane, exact, nullptr, 0);
         float* x = ws + L.x;
         float* g = ws + L.g;
         for (int i = lane; i < SDM; i += 32) x[i] = state[(long long)ch * SDM + i];

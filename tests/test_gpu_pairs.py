@@ -1,0 +1,61 @@
+"""The intra-pair loop of the search kernels: how the slots of a round are linked (adock_prepare), and energies and
+gradients of ligands whose rounds repeat atoms the most (few atoms, one rotatable bond) or fill every atom bucket,
+against the oracle's C restatement at the parity bar of test_gpu_parity.py (1e-4)."""
+import numpy as np
+import pytest
+import torch
+
+from helpers import lig_types, make_problem, random_states, receptor, rel_close, vec_rel, SPACING
+
+pytestmark = pytest.mark.gpu
+DEV = torch.device("cuda:0")
+SIZES = [(4, 1), (6, 1), (8, 2), (12, 1), (31, 6), (32, 1), (33, 9), (64, 12), (65, 10), (96, 8), (100, 16)]
+
+
+def _problems(n_heavy, n_rot):
+    from adock_b200 import params, synth
+    from adock_b200.grid import build_grid, grid_dims
+    sfp = params.sf_params("vina")
+    rec = receptor("small")
+    ligs = [synth.ligand(n_heavy, n_rot, 40 + n_heavy)]
+    lt = lig_types(ligs)
+    o = rec["center"] - rec["size"] / 2
+    G = build_grid(rec["rec_xyz"], rec["rec_types"], sfp, o, SPACING, grid_dims(rec["size"], SPACING), lt,
+                   device=DEV).cpu().numpy()
+    return make_problem(rec, ligs, sfp, G, lt, DEV), make_problem(rec, ligs, sfp, G, lt, "cpu")
+
+
+@pytest.mark.parametrize("n_heavy,n_rot", SIZES)
+def test_rounds_are_linked_in_lane_order(n_heavy, n_rot):
+    from adock_b200.kernel import B200KernelProblem
+    pg, _ = _problems(n_heavy, n_rot)
+    kp = B200KernelProblem(pg)
+    rec = kp.t_work[3].view(-1, 32, 2).cpu().numpy()
+    for x, y in zip(rec[:, :, 0], rec[:, :, 1]):
+        lanes = np.flatnonzero(x >= 0)
+        for side in (0, 1):
+            atom = (x >> (8 * side)) & 0xff
+            most = 0
+            for a in np.unique(atom[lanes]):
+                chain = [k for k in lanes if atom[k] == a]
+                want = dict(zip(chain, chain[1:] + chain[-1:]))
+                assert all((x[k] >> (18 + 5 * side)) & 31 == want[k] for k in chain)
+                assert [(x[k] >> (28 + side)) & 1 for k in chain] == [1] + [0] * (len(chain) - 1)
+                most = max(most, len(chain) - 1)
+            if len(lanes):
+                assert ((y >> (5 * side)) & 31 == most).all()
+
+
+@pytest.mark.parametrize("n_heavy,n_rot", SIZES)
+def test_energy_and_gradient_over_atom_buckets(n_heavy, n_rot):
+    from adock_b200.kernel import B200KernelProblem
+    from oracle.port import PortProblem
+    pg, pc = _problems(n_heavy, n_rot)
+    kp = B200KernelProblem(pg)
+    cl, st = random_states(pc, 16, seed=n_heavy)
+    for exact in (False, True):
+        e, g = kp.energy_grad(torch.as_tensor(cl, device=DEV), torch.as_tensor(st, device=DEV), exact=exact)
+        ec, gc = PortProblem.from_problem(pc).energy_grad(cl, st, exact=exact)
+        D = 6 + pc.lb.preps[0].n_tors
+        assert rel_close(e.cpu().numpy(), ec) < 1e-4
+        assert vec_rel(g.cpu().numpy()[:, :D], gc[:, :D]) < 1e-4
