@@ -132,6 +132,12 @@ __device__ __forceinline__ float pair_energy(float r, float rsum, int flags, con
     return e;
 }
 
+// The energy of pair_energy alone (same operations, same order).
+__device__ __forceinline__ float pair_energy(float r, float rsum, int flags, const PairPrm& p) {
+    float de;
+    return pair_energy(r, rsum, flags, p, de);
+}
+
 // float64 variant (final re-score)
 __device__ __forceinline__ double pair_energy64(double r, double rsum, int flags, const float* prm) {
     double d = r - rsum;

@@ -28,6 +28,8 @@ namespace adock {
 #define PR_NEXT 18    // + 5 * side
 #define PR_LEAD 28    // + side
 
+#define EX_TILE 64   // receptor atoms that the exact energy stages at a time (one bit each in a 64-bit mask)
+
 struct SearchParams {
     // B200 working layout
     const float4* atoms;   // [L, AM]
@@ -116,13 +118,15 @@ __device__ __forceinline__ void stage_tables(TypeTables& dst, const TypeTables& 
 // ------------------------------------------------------------------------------------------ per-warp workspace
 // Float offsets of the per-warp shared workspace for a given AM / KM (float4 arrays first).
 struct WSLayout {
-    int X, FT, ap, au, tp, tu, ax, cs, sn, H, x, xn, xo, cur, best, g, gn, go, p, y, mhy, total;
-    __host__ __device__ WSLayout(int AM, int KM) {
+    int X, FT, RT, V, ap, au, tp, tu, ax, cs, sn, H, x, xn, xo, cur, best, g, gn, go, total;
+    __host__ __device__ WSLayout(int AM, int KM, bool exact) {
         const int DM = 6 + KM, SD = 7 + KM;
         int o = 0;
         X = o; o += 4 * AM;    // world coordinates and radii, [4][AM] (x, y, z, radius arrays)
         FT = o; o += 8 * AM;   // forces of the pair loop, [3][AM]; then float4 (force, torsion bitmask) and float4
                                // (torque, 0) per atom
+        RT = o; o += exact ? 4 * EX_TILE : 0;   // a tile of receptor atoms, float4 (xyz, type | flags << 8)
+        V = o; o += 4 * DM;    // BFGS vectors, float4 (p, -H y, y, g) per component
         ap = o; o += 4 * KM;
         au = o; o += 4 * KM;
         tp = o; o += 4 * KM;
@@ -139,9 +143,6 @@ struct WSLayout {
         g = o; o += DM;
         gn = o; o += DM;
         go = o; o += DM;
-        p = o; o += DM;
-        y = o; o += DM;
-        mhy = o; o += DM;
         total = (o + 3) & ~3;  // keep 16-byte alignment of the next warp
     }
 };
@@ -254,7 +255,7 @@ __device__ __forceinline__ float trilinear(const GT* G, int ny, int nz, const fl
 // the cutoff. Positions and radii are four arrays of AM floats, so that 32 lanes touching 32 different atoms hit 32
 // different shared-memory banks (a float4 per atom would put the x components of 32 atoms on 8 banks). Branch-free, so
 // that the slots a lane has in flight overlap.
-template <int AM>
+template <int AM, bool GRAD>
 __device__ __forceinline__ float pair_slot(int w, bool valid, const float* X, const PairPrm& pp, float3& f) {
     const float *Xi = X + (w & 0xff), *Xj = X + ((w >> 8) & 0xff);
     const float rx = Xi[0] - Xj[0], ry = Xi[AM] - Xj[AM], rz = Xi[2 * AM] - Xj[2 * AM];
@@ -265,8 +266,10 @@ __device__ __forceinline__ float pair_slot(int w, bool valid, const float* X, co
     const bool on = valid && !(r >= pp.cutoff);
     float de;
     const float e = pair_energy(r, Xi[3 * AM] + Xj[3 * AM], w >> 16, pp, de);
-    const float sc = on ? de * rinv : 0.f;
-    f.x = __fmul_rn(sc, rx); f.y = __fmul_rn(sc, ry); f.z = __fmul_rn(sc, rz);
+    if (GRAD) {
+        const float sc = on ? de * rinv : 0.f;
+        f.x = __fmul_rn(sc, rx); f.y = __fmul_rn(sc, ry); f.z = __fmul_rn(sc, rz);
+    }
     return on ? e : 0.f;
 }
 
@@ -306,23 +309,25 @@ __device__ __forceinline__ void push_forces(int w, int repeats, float3 f, float*
     __syncwarp();
 }
 
-// Intra-ligand pairs: adds the lane's slots to its share e of the energy (returned) and the forces on the lane's atoms
-// (lane + 32 i) to F. An atom's contributions are added in the order round, first atoms before second atoms, lane.
+// Intra-ligand pairs: adds the lane's slots to its share e of the energy (returned) and, with GRAD, the forces on the
+// lane's atoms (lane + 32 i) to F. An atom's contributions are added in the order round, first atoms before second atoms, lane.
 // Bound by instruction issue and the latency of the rounds' shared-memory updates (about 95 instructions per slot for
 // the pair term, 66 per round for the two sides). With shared float atomics for the forces and the pair parameters read
 // through a generic pointer this loop took 10.3 k of a single warp's 19 k cycles per evaluation (24 atoms, 7 rounds);
-// now 4.3 k. Summing in registers instead was slower: owners pulling by shuffles (132 instructions per round), or
+// now 2.9 k (averaged over evaluations with and without the gradient). Summing in registers instead was slower: owners pulling by shuffles (132 instructions per round), or
 // per-atom slot lists over forces left in shared memory (12 wavefronts per entry from bank conflicts).
-template <int APL>
+template <int APL, bool GRAD>
 __device__ __forceinline__ float pair_terms(float* ws, const WSLayout& L, const Chain<APL>& c, const PairPrm& pp,
                                             float3 (&F)[APL], float e, int lane) {
     constexpr int AM = 32 * APL;
     const float* X = ws + L.X;
     float* FF = ws + L.FT;
+    if (GRAD) {
 #pragma unroll
-    for (int i = 0; i < APL; ++i) {
-        const int a = lane + 32 * i;
-        FF[a] = F[i].x; FF[AM + a] = F[i].y; FF[2 * AM + a] = F[i].z;
+        for (int i = 0; i < APL; ++i) {
+            const int a = lane + 32 * i;
+            FF[a] = F[i].x; FF[AM + a] = F[i].y; FF[2 * AM + a] = F[i].z;
+        }
     }
     __syncwarp();
     // two rounds in flight; the next two rounds' records are loaded while these are evaluated
@@ -336,24 +341,112 @@ __device__ __forceinline__ float pair_terms(float* ws, const WSLayout& L, const 
         const int2 qb = (r + 3 < c.nrounds) ? c.pairs[(r + 3) * 32 + lane] : none;
         const int wa = pa.x < 0 ? empty : pa.x, wb = pb.x < 0 ? empty : pb.x;
         float3 fa, fb;
-        e += pair_slot<AM>(wa, pa.x >= 0, X, pp, fa);
-        e += pair_slot<AM>(wb, pb.x >= 0, X, pp, fb);
-        push_forces<AM, 0>(wa, pa.y & 31, fa, FF);
-        push_forces<AM, 1>(wa, pa.y >> 5, fa, FF);
-        if (r + 1 < c.nrounds) {
-            push_forces<AM, 0>(wb, pb.y & 31, fb, FF);
-            push_forces<AM, 1>(wb, pb.y >> 5, fb, FF);
+        e += pair_slot<AM, GRAD>(wa, pa.x >= 0, X, pp, fa);
+        e += pair_slot<AM, GRAD>(wb, pb.x >= 0, X, pp, fb);
+        if (GRAD) {
+            push_forces<AM, 0>(wa, pa.y & 31, fa, FF);
+            push_forces<AM, 1>(wa, pa.y >> 5, fa, FF);
+            if (r + 1 < c.nrounds) {
+                push_forces<AM, 0>(wb, pb.y & 31, fb, FF);
+                push_forces<AM, 1>(wb, pb.y >> 5, fb, FF);
+            }
         }
         pa = qa;
         pb = qb;
     }
+    if (GRAD) {
 #pragma unroll
-    for (int i = 0; i < APL; ++i) {
-        const int a = lane + 32 * i;
-        F[i] = make_float3(FF[a], FF[AM + a], FF[2 * AM + a]);
+        for (int i = 0; i < APL; ++i) {
+            const int a = lane + 32 * i;
+            F[i] = make_float3(FF[a], FF[AM + a], FF[2 * AM + a]);
+        }
     }
     __syncwarp();
     return e;
+}
+
+// Exact inter energy of the lane's atoms (positions in shared memory) with the receptor atoms, or the chain's
+// neighbour list: sums in list order, and with `grad` the forces into F. A tile of receptor atoms is staged in shared
+// memory; each lane first collects the tile's atoms inside the cutoff of its atom as a bit mask (a few instructions per
+// pair, no branches), then evaluates the pair terms of its set bits, two in flight, so that the terms run with most
+// lanes busy: some 50 of a pose's 300 neighbours are inside the 8 A cutoff of one atom. Bound by instruction issue.
+// Walking the list with dependent loads and evaluating the terms wherever any lane's pair was inside took 190 k cycles
+// per evaluation (300 neighbours, 14 warps per SM), this about 31 k.
+template <int APL>
+__device__ __forceinline__ void exact_terms(float* ws, const WSLayout& L, const Chain<APL>& c, const SearchParams& P,
+                                            const TypeTables& tt, float (&inter)[APL], float3 (&F)[APL], int lane,
+                                            bool grad) {
+    constexpr int AM = 32 * APL;
+    const float* X = ws + L.X;
+    float4* RT = (float4*)(ws + L.RT);
+    const float cut2 = P.pp.cutoff * P.pp.cutoff;
+    const int n = c.nb ? c.nbn : c.rn;
+    auto fetch = [&](int k) {
+        if (k >= n) return make_float4(0.f, 0.f, 0.f, 0.f);
+        const int b = c.nb ? c.nb[k] : k;
+        const int tb = c.rt[b] & 63;   // index kept inside the 64-entry type tables
+        return make_float4(c.rx[3 * b], c.rx[3 * b + 1], c.rx[3 * b + 2], __int_as_float(tb | (tt.flags[tb] << 8)));
+    };
+#pragma unroll
+    for (int i = 0; i < APL; ++i) inter[i] = 0.f;
+    float4 n0 = fetch(lane), n1 = fetch(32 + lane);
+#pragma unroll 1
+    for (int t0 = 0; t0 < n; t0 += EX_TILE) {
+        __syncwarp();
+        RT[lane] = n0;
+        RT[32 + lane] = n1;
+        __syncwarp();
+        n0 = fetch(t0 + EX_TILE + lane);
+        n1 = fetch(t0 + EX_TILE + 32 + lane);
+        const unsigned long long valid = n - t0 >= 64 ? ~0ull : (1ull << (n - t0)) - 1ull;
+#pragma unroll
+        for (int i = 0; i < APL; ++i) {
+            if (32 * i >= c.na) break;
+            const int a = lane + 32 * i;
+            const float X0 = X[a], X1 = X[AM + a], X2 = X[2 * AM + a];
+            unsigned m0 = 0, m1 = 0;
+#pragma unroll 8
+            for (int b = 0; b < 32; ++b) {
+                const float4 B = RT[b], C = RT[32 + b];
+                float rx = X0 - B.x, ry = X1 - B.y, rz = X2 - B.z;
+                float r2 = rx * rx + ry * ry + rz * rz;
+                m0 |= (r2 >= cut2 ? 0u : 1u) << b;
+                rx = X0 - C.x; ry = X1 - C.y; rz = X2 - C.z;
+                r2 = rx * rx + ry * ry + rz * rz;
+                m1 |= (r2 >= cut2 ? 0u : 1u) << b;
+            }
+            unsigned long long m = a < c.na ? (((unsigned long long)m1 << 32) | m0) & valid : 0ull;
+            const int ta = c.typ[i] & 63;
+            const float ra = tt.radius[ta];
+            const int fa = tt.flags[ta];
+            float ea = inter[i];
+            float3 f = F[i];
+            const int most = __reduce_max_sync(0xffffffffu, __popcll(m));
+#pragma unroll 1
+            for (int t = 0; t < most; t += 2) {
+#pragma unroll
+                for (int u = 0; u < 2; ++u) {
+                    const bool on = m != 0ull;
+                    const float4 B = RT[on ? __ffsll((long long)m) - 1 : 0];
+                    m &= m - 1ull;
+                    const float rx = X0 - B.x, ry = X1 - B.y, rz = X2 - B.z;
+                    const float r2 = rx * rx + ry * ry + rz * rz;
+                    const int tb = __float_as_int(B.w) & 63, fb = __float_as_int(B.w) >> 8;
+                    const float rinv = rsqrt_ftz(fmaxf(r2, 1e-12f));
+                    const float r = r2 * rinv;
+                    float de;
+                    const float ep = pair_energy(r, ra + tt.radius[tb], hyd_pair(fa, fb) | hb_pair(fa, fb), P.pp, de);
+                    if (on) {
+                        ea += ep;
+                        const float sc = de * rinv;
+                        f.x += sc * rx; f.y += sc * ry; f.z += sc * rz;
+                    }
+                }
+            }
+            inter[i] = ea;
+            F[i] = f;
+        }
+    }
 }
 
 // Energy + analytic pose gradient of state s (shared, SD floats) into g (shared, DM floats); E on all lanes.
@@ -362,10 +455,11 @@ __device__ __forceinline__ float pair_terms(float* ws, const WSLayout& L, const 
 // pairs. Gradient: dE/dt = sum F, torque = sum (X - t) x F, dE/dtheta_k = u_k . sum_{a moved by k} (X_a - p_k) x F_a,
 // evaluated as u_k . (sum X' x F - p'_k x sum F) over the subtree of k (X' = X - t).
 // EX selects the inter energy at compile time: exact pairwise over receptor atoms (or the chain's neighbour list),
-// else the trilinear grid, so the grid-mode kernels carry no receptor loop.
+// else the trilinear grid, so the grid-mode kernels carry no receptor loop. Without `grad` only the energy is
+// evaluated (the same value) and g is left alone: a rejected line-search point needs no gradient.
 template <int APL, typename GT, bool EX>
 __device__ __forceinline__ float eval_eg(float* ws, const WSLayout& L, const float* s, float* g, const Chain<APL>& c,
-                         const SearchParams& P, const TypeTables& tt, int lane) {
+                         const SearchParams& P, const TypeTables& tt, int lane, bool grad) {
     constexpr int AM = 32 * APL;
     float* X = ws + L.X;     // [3][AM] world coordinates (radii behind them)
     const float4* ap = (const float4*)(ws + L.ap);
@@ -392,6 +486,7 @@ __device__ __forceinline__ float eval_eg(float* ws, const WSLayout& L, const flo
     __syncwarp();
     float e = 0.f;
     float3 F[APL];   // dE/dX of the lane's atoms
+    float inter[APL];
     const GT* grid = (const GT*)c.grid;
 #pragma unroll
     for (int i = 0; i < APL; ++i) {
@@ -418,29 +513,18 @@ __device__ __forceinline__ float eval_eg(float* ws, const WSLayout& L, const flo
             X[a] = X0;
             X[AM + a] = X1;
             X[2 * AM + a] = X2;
+        }
+    }
+    if constexpr (EX) exact_terms<APL>(ws, L, c, P, tt, inter, F, lane, grad);
+#pragma unroll
+    for (int i = 0; i < APL; ++i) {
+        const int a = lane + 32 * i;
+        if (a < c.na) {
+            const float X0 = X[a], X1 = X[AM + a], X2 = X[2 * AM + a];
             float ea, gg[3];
             if constexpr (EX) {
-                ea = 0.f;
-                gg[0] = gg[1] = gg[2] = 0.f;
-                const int ta = c.typ[i] & 63;
-                const float ra = tt.radius[ta];
-                const int fa = tt.flags[ta];
-                const float cut2 = P.pp.cutoff * P.pp.cutoff;
-                const int nloop = c.nb ? c.nbn : c.rn;
-                for (int bb = 0; bb < nloop; ++bb) {
-                    const int b = c.nb ? c.nb[bb] : bb;
-                    const float rx = X0 - c.rx[3 * b], ry = X1 - c.rx[3 * b + 1], rz = X2 - c.rx[3 * b + 2];
-                    const float r2 = rx * rx + ry * ry + rz * rz;
-                    if (r2 >= cut2) continue;
-                    const int tb = c.rt[b] & 63;   // index kept inside the 64-entry type tables
-                    const int fb = tt.flags[tb];
-                    const float rinv = rsqrtf(fmaxf(r2, 1e-12f));
-                    const float r = r2 * rinv;
-                    float de;
-                    ea += pair_energy(r, ra + tt.radius[tb], hyd_pair(fa, fb) | hb_pair(fa, fb), P.pp, de);
-                    const float sc = de * rinv;
-                    gg[0] += sc * rx; gg[1] += sc * ry; gg[2] += sc * rz;
-                }
+                ea = inter[i];
+                gg[0] = F[i].x; gg[1] = F[i].y; gg[2] = F[i].z;
             } else {
                 ea = trilinear<GT>(grid + (long long)c.slot[i] * c.n3, c.ny, c.nz, c.o, c.fmx, P.inv_s, X0, X1, X2,
                                    gg[0], gg[1], gg[2]);
@@ -457,7 +541,12 @@ __device__ __forceinline__ float eval_eg(float* ws, const WSLayout& L, const flo
         }
     }
     __syncwarp();
-    e = pair_terms<APL>(ws, L, c, P.pp, F, e, lane);
+    if (!grad) {
+        e = warp_sum(pair_terms<APL, false>(ws, L, c, P.pp, F, e, lane));
+        __syncwarp();
+        return e;
+    }
+    e = pair_terms<APL, true>(ws, L, c, P.pp, F, e, lane);
     // world torsion axes (axis atoms' current positions)
     for (int k = lane; k < c.nt; k += 32) {
         const int a0 = axs[k] & 0xffff, a1 = axs[k] >> 16;
@@ -540,43 +629,32 @@ __device__ __forceinline__ float eval_eg(float* ws, const WSLayout& L, const flo
     return e;
 }
 
-__device__ __forceinline__ float wdot(const float* a, const float* b, int D, int lane) {
-    float s = 0.f;
-    for (int i = lane; i < D; i += 32) s += a[i] * b[i];
-    return warp_sum(s);
-}
-__device__ __forceinline__ double wdot64(const float* a, const float* b, int D, int lane) {
-    double s = 0.0;
-    for (int i = lane; i < D; i += 32) s += (double)a[i] * (double)b[i];
-    return warp_sum_d(s);
-}
 __device__ __forceinline__ void wcopy(float* dst, const float* src, int D, int lane) {
     for (int i = lane; i < D; i += 32) dst[i] = src[i];
     __syncwarp();
 }
-// xn = x (+) alpha p: translation add, rotation-vector increment of the quaternion, torsion add (mckernel.py:256-265)
-__device__ __forceinline__ void conf_step(float* xn, const float* x, const float* p, float alpha, int nt, int lane) {
+// xn = x (+) alpha p (p = V[].x): translation add, rotation-vector increment of the quaternion, torsion add (mckernel.py:256-265)
+__device__ __forceinline__ void conf_step(float* xn, const float* x, const float4* V, float alpha, int nt, int lane) {
     if (lane == 0) {
-        xn[0] = x[0] + alpha * p[0]; xn[1] = x[1] + alpha * p[1]; xn[2] = x[2] + alpha * p[2];
+        xn[0] = x[0] + alpha * V[0].x; xn[1] = x[1] + alpha * V[1].x; xn[2] = x[2] + alpha * V[2].x;
         xn[3] = x[3]; xn[4] = x[4]; xn[5] = x[5]; xn[6] = x[6];
-        quat_apply_rotvec(xn + 3, alpha * p[3], alpha * p[4], alpha * p[5]);
+        quat_apply_rotvec(xn + 3, alpha * V[3].x, alpha * V[4].x, alpha * V[5].x);
     }
-    for (int k = lane; k < nt; k += 32) xn[7 + k] = x[7 + k] + alpha * p[6 + k];
+    for (int k = lane; k < nt; k += 32) xn[7 + k] = x[7 + k] + alpha * V[6 + k].x;
     __syncwarp();
 }
-// out_i = -sum_j H_ij v_j; H symmetric, stored with lane i owning column i (conflict-free); two accumulators
-__device__ __forceinline__ void neg_hv(const float* H, const float* v, float* out, int D, int lane) {
-    for (int i = lane; i < D; i += 32) {
-        float a0 = 0.f, a1 = 0.f;
-        int j = 0;
-        for (; j + 1 < D; j += 2) {
-            a0 += H[j * D + i] * v[j];
-            a1 += H[(j + 1) * D + i] * v[j + 1];
-        }
-        if (j < D) a0 += H[j * D + i] * v[j];
-        out[i] = -(a0 + a1);
+// -sum_j H_ij v_j of component i (component `v` of the vectors V); H symmetric, stored with lane i owning column i
+// (conflict-free); two accumulators
+template <int v>
+__device__ __forceinline__ float neg_hv(const float* H, const float4* V, int i, int D) {
+    float a0 = 0.f, a1 = 0.f;
+    int j = 0;
+    for (; j + 1 < D; j += 2) {
+        a0 += H[j * D + i] * (v == 2 ? V[j].z : V[j].w);
+        a1 += H[(j + 1) * D + i] * (v == 2 ? V[j + 1].z : V[j + 1].w);
     }
-    __syncwarp();
+    if (j < D) a0 += H[j * D + i] * (v == 2 ? V[j].z : V[j].w);
+    return -(a0 + a1);
 }
 
 // Vina-1.2-style BFGS on state x (shared, in/out); returns the final energy (mckernel.py:267-326).
@@ -592,81 +670,135 @@ __device__ __forceinline__ float bfgs(float* ws, const WSLayout& L, float* x, in
     float* g = ws + L.g;
     float* gn = ws + L.gn;
     float* go = ws + L.go;
-    float* p = ws + L.p;
-    float* y = ws + L.y;
-    float* mhy = ws + L.mhy;
+    float4* V = (float4*)(ws + L.V);
     float* xn = ws + L.xn;
     float* xo = ws + L.xo;
     // One evaluation per pass of this loop: the start point on the first pass, then the line-search trial points.
-    // Keeping a single call site keeps a single inlined copy of eval_eg in the kernel.
+    // Keeping a single call site keeps a single inlined copy of eval_eg in the kernel. About 70 % of the first trials
+    // are accepted, but only a third of the later ones: those are evaluated without the gradient first, and once more
+    // with it (`again`, the same energy) when they are accepted. The 10th point is taken in any case.
     float f0 = 0.f, f_orig = 0.f, pg = 0.f, alpha = 1.f;
     int step = 0, trial = 0;
-    bool first = true;
+    bool first = true, again = false;
     while (true) {
-        const float f = eval_eg<APL, GT, EX>(ws, L, first ? x : xn, first ? g : gn, c, P, tt, lane);
-        ++n_eval;
+        const bool grad = first || again || trial == 0 || trial == 9;
+        const float f = eval_eg<APL, GT, EX>(ws, L, first ? x : xn, first ? g : gn, c, P, tt, lane, grad);
+        if (!again) ++n_eval;
         if (first) {
             first = false;
             f0 = f_orig = f;
             wcopy(xo, x, S, lane);
-            wcopy(go, g, D, lane);
-            for (int i = lane; i < D; i += 32)
-                for (int j = 0; j < D; ++j) H[j * D + i] = (i == j) ? 1.f : 0.f;
+            float s = 0.f;
+            for (int i = lane; i < D; i += 32) {
+                go[i] = g[i];
+                float a0 = 0.f, a1 = 0.f;   // p = -H g with H the identity
+                for (int j = 0; j < D; ++j) (j & 1 ? a1 : a0) += (i == j ? 1.f : 0.f) * g[j];
+                const float pi = -(a0 + a1);
+                V[i].x = pi;
+                s += pi * g[i];
+            }
             __syncwarp();
             if (iters <= 0) break;
-            neg_hv(H, g, p, D, lane);
-            pg = wdot(p, g, D, lane);
-            alpha = 1.f;
-            trial = 0;
-            conf_step(xn, x, p, alpha, c.nt, lane);
+            pg = warp_sum(s);
+            conf_step(xn, x, V, alpha, c.nt, lane);
             continue;
         }
         // Armijo test (c = 1e-4); up to 10 trials halving alpha. After a 10th failed trial the last point is taken
         // with alpha already halved, as in the reference's loop.
-        if (!(f - f0 < 1e-4f * alpha * pg)) {
-            alpha *= 0.5f;
-            if (++trial < 10) {
-                conf_step(xn, x, p, alpha, c.nt, lane);
+        bool stuck = false;
+        if (!again) {
+            if (!(f - f0 < 1e-4f * alpha * pg)) {
+                alpha *= 0.5f;
+                if (++trial < 10) {
+                    conf_step(xn, x, V, alpha, c.nt, lane);
+                    continue;
+                }
+                stuck = true;
+                for (int i = lane; i < S; i += 32) stuck = stuck && __float_as_int(x[i]) == __float_as_int(xn[i]);
+                stuck = __all_sync(0xffffffffu, stuck);
+            } else if (!grad) {
+                again = true;
                 continue;
             }
         }
-        for (int i = lane; i < D; i += 32) y[i] = gn[i] - g[i];
-        __syncwarp();
+        again = false;
+        // The 10th point is the iteration's own start: its gradient step is 0, H stays, and every further iteration
+        // would repeat this one.
+        if (stuck) break;
         f0 = f;
-        wcopy(x, xn, S, lane);
-        const float gg = wdot(gn, gn, D, lane);
-        wcopy(g, gn, D, lane);
+        for (int i = lane; i < S; i += 32) x[i] = xn[i];
+        float gg = 0.f, yy = 0.f;
+        double yp = 0.0;
+        for (int i = lane; i < D; i += 32) {
+            const float gi = gn[i], yi = gi - g[i];
+            gg += gi * gi;
+            yy += yi * yi;
+            yp += (double)yi * (double)V[i].x;
+            g[i] = gi;
+            V[i].z = yi;
+            V[i].w = gi;
+        }
+        __syncwarp();
+        gg = warp_sum(gg);
+        yy = warp_sum(yy);
+        yp = warp_sum_d(yp);
         if (!(sqrtf(gg) >= 1e-5f)) break;
-        const double yp = wdot64(y, p, D, lane);
-        if (step == 0) {
-            const float yy = wdot(y, y, D, lane);
-            if (fabsf(yy) > EPSF) {
-                const float dg = (float)((double)alpha * yp / (double)yy);
-                for (int i = lane; i < D; i += 32)
-                    for (int j = 0; j < D; ++j) H[j * D + i] = (i == j) ? dg : 0.f;
-                __syncwarp();
-            }
+        if (step == 0) {   // H: the identity, rescaled from the first step's curvature
+            const float dg = fabsf(yy) > EPSF ? (float)((double)alpha * yp / (double)yy) : 1.f;
+            for (int i = lane; i < D; i += 32)
+                for (int j = 0; j < D; ++j) H[j * D + i] = (i == j) ? dg : 0.f;
+            __syncwarp();
         }
         const double ayp = (double)alpha * yp;
+        float s = 0.f;
         if (ayp >= (double)EPSF) {
-            for (int i = lane; i < D; i += 32) mhy[i] = 0.f;
-            neg_hv(H, y, mhy, D, lane);
-            const float yhy = -wdot(y, mhy, D, lane);
+            for (int i = lane; i < D; i += 32) {
+                const float mi = neg_hv<2>(H, V, i, D);
+                V[i].y = mi;
+                s += V[i].z * mi;
+            }
+            __syncwarp();
+            const float yhy = -warp_sum(s);
             const float r = (float)(1.0 / ayp);
             const float c2 = alpha * alpha * (r * r * yhy + r);
             const float ar = alpha * r;
-            for (int i = lane; i < D; i += 32) {
-                const float mi = mhy[i], pi = p[i];
-                for (int j = 0; j < D; ++j) H[j * D + i] += ar * (mi * p[j] + mhy[j] * pi) + c2 * pi * p[j];
+            // the update and the new direction -H g in one sweep over H
+            s = 0.f;
+            float pn[2];
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const int i = lane + 32 * h;
+                pn[h] = 0.f;
+                if (i < D) {
+                    const float mi = V[i].y, pi = V[i].x;
+                    float a0 = 0.f, a1 = 0.f;
+                    for (int j = 0; j < D; ++j) {
+                        const float4 v = V[j];
+                        float hij = H[j * D + i];
+                        hij += ar * (mi * v.x + v.y * pi) + c2 * pi * v.x;
+                        H[j * D + i] = hij;
+                        if (j & 1) a1 += hij * v.w; else a0 += hij * v.w;
+                    }
+                    pn[h] = -(a0 + a1);
+                    s += pn[h] * V[i].w;
+                }
             }
             __syncwarp();
+            if (lane < D) V[lane].x = pn[0];
+            if (lane + 32 < D) V[lane + 32].x = pn[1];
+        } else {
+            for (int i = lane; i < D; i += 32) {
+                const float pi = neg_hv<3>(H, V, i, D);
+                s += pi * V[i].w;
+                V[i].x = pi;
+            }
         }
+        __syncwarp();
         if (++step >= iters) break;
-        neg_hv(H, g, p, D, lane);
-        pg = wdot(p, g, D, lane);
+        pg = warp_sum(s);
         alpha = 1.f;
         trial = 0;
-        conf_step(xn, x, p, alpha, c.nt, lane);
+        conf_step(xn, x, V, alpha, c.nt, lane);
     }
     if (!(f0 <= f_orig)) {
         f0 = f_orig;
@@ -808,7 +940,7 @@ __global__ void __launch_bounds__(128, MINB) mc_kernel(const __grid_constant__ S
     __shared__ TypeTables tt;
     stage_tables(tt, ttg);
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    const WSLayout L(P.AM, P.KM);
+    const WSLayout L(P.AM, P.KM, EX);
     float* ws = (float*)smem4 + (size_t)wid * L.total;
     const int SDM = 7 + P.KM;
     unsigned n_eval = 0;
@@ -956,7 +1088,7 @@ __global__ void __launch_bounds__(128) eg_kernel(const __grid_constant__ SearchP
     __shared__ TypeTables tt;
     stage_tables(tt, ttg);
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    const WSLayout L(P.AM, P.KM);
+    const WSLayout L(P.AM, P.KM, EX);
     float* ws = (float*)smem4 + (size_t)wid * L.total;
     const int SDM = 7 + P.KM, DMM = 6 + P.KM;
     const int warps = (blockDim.x >> 5) * gridDim.x;
@@ -968,7 +1100,7 @@ __global__ void __launch_bounds__(128) eg_kernel(const __grid_constant__ SearchP
         float* g = ws + L.g;
         for (int i = lane; i < SDM; i += 32) x[i] = state[(long long)ch * SDM + i];
         __syncwarp();
-        const float e = eval_eg<APL, GT, EX>(ws, L, x, g, c, P, tt, lane);
+        const float e = eval_eg<APL, GT, EX>(ws, L, x, g, c, P, tt, lane, true);
         for (int i = lane; i < 6 + c.nt; i += 32) g_out[(long long)ch * DMM + i] = g[i];
         if (lane == 0) e_out[ch] = e;
         __syncwarp();
@@ -1201,7 +1333,7 @@ static const int MC_VARIANT_MINB[4] = {4, 4, 6, 8};
 template <int APL, typename GT, int MINB>
 static int launch_mc_v(const SearchParams& P, const McParams& M, const TypeTables& tt, cudaStream_t st) {
     const int wpb = 4;
-    const WSLayout L(P.AM, P.KM);
+    const WSLayout L(P.AM, P.KM, M.exact);
     const size_t smem = (size_t)wpb * L.total * sizeof(float);
     auto kern = M.exact ? mc_kernel<APL, GT, MINB, true> : mc_kernel<APL, GT, MINB, false>;
     ADOCK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
@@ -1241,7 +1373,7 @@ template <int APL, typename GT>
 static int launch_eg_t(const SearchParams& P, const int* cl, int n, const float* state, float* e, float* g, int exact,
                        const TypeTables& tt, cudaStream_t st) {
     const int wpb = 4;
-    const WSLayout L(P.AM, P.KM);
+    const WSLayout L(P.AM, P.KM, exact);
     const size_t smem = (size_t)wpb * L.total * sizeof(float);
     auto kern = exact ? eg_kernel<APL, GT, true> : eg_kernel<APL, GT, false>;
     ADOCK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
