@@ -85,6 +85,9 @@ _SIGS = {
     "adock_gemm_bf16_mma": ([I, I, I, P, ctypes.c_longlong, ctypes.c_longlong, P, ctypes.c_longlong,
                              ctypes.c_longlong, P, ctypes.c_longlong, F, P, I, P, P, ctypes.c_longlong, P], I),
     "adock_gemm_status": ([], I),
+    "adock_mlp_forward": ([I, P, SP(P), SP(P), P, P, P, P, P, P], I),
+    "adock_mlp_workspace_bytes": ([I], ctypes.c_size_t),
+    "adock_mlp_loss_grad": ([I, P, P, SP(P), SP(P), I, P, SP(P), SP(P), P, P], I),
     "adock_mlp_nll": ([P, P, I, I, P, P, P], I),
     "adock_silu_backward": ([P, P, ctypes.c_longlong, P, P], I),
     "adock_bias_grad": ([P, I, I, P, P], I),
@@ -95,9 +98,10 @@ EXPORTS = tuple(_SIGS)
 
 _lib = None
 _lock = threading.Lock()
-# kernel launches issued through call() (each launching entry point issues one kernel)
+# kernel launches issued through call(): one per launching entry point, or its count here
 LAUNCHES = [0]
-_NO_LAUNCH = {"adock_version", "adock_last_error", "adock_mc_noalloc_scratch_bytes", "adock_gemm_status"}
+_LAUNCHES = {"adock_version": 0, "adock_last_error": 0, "adock_mc_noalloc_scratch_bytes": 0, "adock_gemm_status": 0,
+             "adock_mlp_workspace_bytes": 0, "adock_mlp_forward": 3, "adock_mlp_loss_grad": 12}
 
 
 def load():
@@ -120,8 +124,8 @@ def call(name, *args):
     """Call an entry point; a non-zero status raises RuntimeError with the library's message."""
     lib = load()
     rc = getattr(lib, name)(*args)
-    if name not in _NO_LAUNCH and rc == 0:
-        LAUNCHES[0] += 1
+    if rc == 0:
+        LAUNCHES[0] += _LAUNCHES.get(name, 1)
     if rc != 0:
         msg = lib.adock_last_error().decode(errors="replace")
         raise RuntimeError(f"{name} failed ({rc}): {msg}")
@@ -137,6 +141,11 @@ def ptr(t):
         return t.ctypes.data
     assert t.is_contiguous(), "tensor must be contiguous"
     return t.data_ptr()
+
+
+def ptr_array(ts):
+    """Host array of the addresses of contiguous tensors."""
+    return (P * len(ts))(*[ptr(t) for t in ts])
 
 
 def stream_ptr(stream=None):

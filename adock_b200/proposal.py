@@ -89,18 +89,14 @@ class ProposalNet:
     def forward(self, x, save=False):
         """x: BF16 [B, 320] -> out FP32 [B, 64] (and saved activations when save)."""
         B = x.shape[0]
+        assert x.dtype == torch.bfloat16 and x.shape[1] == IN
         dev = self.device
-        pre1 = torch.empty(B, HID, device=dev)
-        h1 = torch.empty(B, HID, dtype=torch.bfloat16, device=dev)
-        pre2 = torch.empty(B, HID, device=dev)
-        h2 = torch.empty(B, HID, dtype=torch.bfloat16, device=dev)
+        h1, h2 = (torch.empty(B, HID, dtype=torch.bfloat16, device=dev) for _ in range(2))
+        pre1, pre2 = (torch.empty(B, HID, device=dev) if save else None for _ in range(2))
         out = torch.empty(B, OUT, device=dev)
-        c1 = torch.empty(B, HID, device=dev)
-        c2 = torch.empty(B, HID, device=dev)
         with torch.cuda.device(dev):
-            _gemm(x, (IN, 1), self.Wb[0], (HID, 1), B, HID, IN, C=c1, bias=self.b[0], act=1, pre=pre1, Cb=h1)
-            _gemm(h1, (HID, 1), self.Wb[1], (HID, 1), B, HID, HID, C=c2, bias=self.b[1], act=1, pre=pre2, Cb=h2)
-            _gemm(h2, (HID, 1), self.Wb[2], (OUT, 1), B, OUT, HID, C=out, bias=self.b[2])
+            _lib.call("adock_mlp_forward", B, _lib.ptr(x), _lib.ptr_array(self.Wb), _lib.ptr_array(self.b),
+                      _lib.ptr(pre1), _lib.ptr(h1), _lib.ptr(pre2), _lib.ptr(h2), _lib.ptr(out), _lib.stream_ptr())
         if save:
             return out, (x, pre1, h1, pre2, h2)
         return out
@@ -108,32 +104,16 @@ class ProposalNet:
     def loss_grad(self, x, y):
         """Mean Gaussian NLL of moves y [B, 32] and the parameter gradients (list matching self.params)."""
         B = x.shape[0]
-        dev = self.device
-        out, (x, pre1, h1, pre2, h2) = self.forward(x, save=True)
-        dout = torch.empty(B, OUT, dtype=torch.bfloat16, device=dev)
-        loss = torch.zeros(1, device=dev)
+        assert x.dtype == torch.bfloat16 and x.shape[1] == IN
+        assert y.dtype == torch.float32 and y.shape == (B, 32)
+        loss = torch.empty(1, device=self.device)
         gW = [torch.empty_like(w) for w in self.W]
         gb = [torch.empty_like(b) for b in self.b]
-        dH2 = torch.empty(B, HID, device=dev)
-        dA2 = torch.empty(B, HID, dtype=torch.bfloat16, device=dev)
-        dH1 = torch.empty(B, HID, device=dev)
-        dA1 = torch.empty(B, HID, dtype=torch.bfloat16, device=dev)
-        s = _lib.stream_ptr
-        with torch.cuda.device(dev):
-            _lib.call("adock_mlp_nll", _lib.ptr(out), _lib.ptr(y), B, self.n_comp, _lib.ptr(dout), _lib.ptr(loss), s())
-            # layer 3: dW3 = h2^T dout, db3, dH2 = dout W3^T
-            _gemm(h2, (1, HID), dout, (OUT, 1), HID, OUT, B, C=gW[2])
-            _lib.call("adock_bias_grad", _lib.ptr(dout), B, OUT, _lib.ptr(gb[2]), s())
-            _gemm(dout, (OUT, 1), self.Wb[2], (1, OUT), B, HID, OUT, C=dH2)
-            _lib.call("adock_silu_backward", _lib.ptr(dH2), _lib.ptr(pre2), B * HID, _lib.ptr(dA2), s())
-            # layer 2
-            _gemm(h1, (1, HID), dA2, (HID, 1), HID, HID, B, C=gW[1])
-            _lib.call("adock_bias_grad", _lib.ptr(dA2), B, HID, _lib.ptr(gb[1]), s())
-            _gemm(dA2, (HID, 1), self.Wb[1], (1, HID), B, HID, HID, C=dH1)
-            _lib.call("adock_silu_backward", _lib.ptr(dH1), _lib.ptr(pre1), B * HID, _lib.ptr(dA1), s())
-            # layer 1
-            _gemm(x, (1, IN), dA1, (HID, 1), IN, HID, B, C=gW[0])
-            _lib.call("adock_bias_grad", _lib.ptr(dA1), B, HID, _lib.ptr(gb[0]), s())
+        work = torch.empty(_lib.load().adock_mlp_workspace_bytes(B), dtype=torch.uint8, device=self.device)
+        with torch.cuda.device(self.device):
+            _lib.call("adock_mlp_loss_grad", B, _lib.ptr(x), _lib.ptr(y), _lib.ptr_array(self.Wb),
+                      _lib.ptr_array(self.b), self.n_comp, _lib.ptr(work), _lib.ptr_array(gW), _lib.ptr_array(gb),
+                      _lib.ptr(loss), _lib.stream_ptr())
         return loss / B, gW + gb
 
     def train_step(self, x, y, lr=1e-3, wd=0.0):

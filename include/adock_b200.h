@@ -313,6 +313,17 @@ int adock_gemm_bf16_mma(int M, int N, int K, const void* A, long long sAm, long 
 /* Device status of the tcgen05 GEMMs since the last call (synchronises): ADOCK_E_DEVICE if a CTA gave up waiting
  * for its tensor-core work (its tile is then not written), else 0. Clears the status. */
 int adock_gemm_status(void);
+/* The network's forward pass on x (BF16 [B, 320]): W (host array of 3 dev pointers) = BF16 weights [320, 256],
+ * [256, 256], [256, 64] row-major, b (host array of 3) = FP32 biases. h1, h2 (BF16 [B, 256], dev) receive the hidden
+ * activations, pre1, pre2 (FP32 [B, 256]; NULL: not kept) the pre-activations, out (FP32 [B, 64]) the output. Queues
+ * the three adock_gemm_bf16 products. */
+int adock_mlp_forward(int B, const void* x, const void* const* W, const float* const* b, float* pre1, void* h1,
+                      float* pre2, void* h2, float* out, void* stream);
+/* Forward pass, adock_mlp_nll and backward pass of a batch: *loss = summed NLL of target [B, 32], gW, gb (host arrays
+ * of 3 dev pointers, FP32) = gradients of the batch mean. work: dev, adock_mlp_workspace_bytes(B), 256-byte aligned. */
+size_t adock_mlp_workspace_bytes(int B);
+int adock_mlp_loss_grad(int B, const void* x, const float* target, const void* const* W, const float* const* b,
+                        int n_comp, void* work, float* const* gW, float* const* gb, float* loss, void* stream);
 /* Gaussian NLL of moves target [B, 32] under out [B, 64]; dout (BF16 [B, 64]) = gradient of the batch mean;
  * *loss += summed NLL. n_comp = 3: the translation term is a 3-component mixture (layout as adock_prop_sample). */
 int adock_mlp_nll(const float* out, const float* target, int B, int n_comp, void* dout, float* loss, void* stream);
