@@ -138,21 +138,31 @@ __device__ __forceinline__ float pair_energy(float r, float rsum, int flags, con
     return pair_energy(r, rsum, flags, p, de);
 }
 
-// float64 variant (final re-score)
-__device__ __forceinline__ double pair_energy64(double r, double rsum, int flags, const float* prm) {
-    double d = r - rsum;
-    double u1 = (d - (double)prm[0]) / (double)prm[1], u2 = (d - (double)prm[2]) / (double)prm[3];
-    double e = (double)prm[10] * exp(-u1 * u1) + (double)prm[11] * exp(-u2 * u2);
-    double dr = d - (double)prm[4];
-    if (dr < 0.0) e += (double)prm[12] * dr * dr;
-    if (flags & PF_HYD) {
-        double v = ((double)prm[6] - d) / ((double)prm[6] - (double)prm[5]);
-        e += (double)prm[13] * fmin(fmax(v, 0.0), 1.0);
-    }
-    if (flags & PF_HB) {
-        double v = ((double)prm[8] - d) / ((double)prm[8] - (double)prm[7]);
-        e += (double)prm[14] * fmin(fmax(v, 0.0), 1.0);
-    }
+// float64 variant (final re-score), with the widths' reciprocals in place of a division per term
+struct PairPrm64 {
+    double g1_off, g1_inv, g2_off, g2_inv, rep_off, hyd_bad, hyd_inv, hb_bad, hb_inv, cutoff;
+    double w_g1, w_g2, w_rep, w_hyd, w_hb;
+};
+
+__host__ inline PairPrm64 make_pair_prm64(const float* prm) {
+    PairPrm64 p;
+    p.g1_off = prm[0]; p.g1_inv = 1.0 / (double)prm[1]; p.g2_off = prm[2]; p.g2_inv = 1.0 / (double)prm[3];
+    p.rep_off = prm[4];
+    p.hyd_bad = prm[6]; p.hyd_inv = 1.0 / ((double)prm[6] - (double)prm[5]);
+    p.hb_bad = prm[8]; p.hb_inv = 1.0 / ((double)prm[8] - (double)prm[7]);
+    p.cutoff = prm[9];
+    p.w_g1 = prm[10]; p.w_g2 = prm[11]; p.w_rep = prm[12]; p.w_hyd = prm[13]; p.w_hb = prm[14];
+    return p;
+}
+
+__device__ __forceinline__ double pair_energy64(double r, double rsum, int flags, const PairPrm64& p) {
+    const double d = r - rsum;
+    const double u1 = (d - p.g1_off) * p.g1_inv, u2 = (d - p.g2_off) * p.g2_inv;
+    double e = p.w_g1 * exp(-u1 * u1) + p.w_g2 * exp(-u2 * u2);
+    const double dr = d - p.rep_off;
+    if (dr < 0.0) e += p.w_rep * dr * dr;
+    if (flags & PF_HYD) e += p.w_hyd * fmin(fmax((p.hyd_bad - d) * p.hyd_inv, 0.0), 1.0);
+    if (flags & PF_HB) e += p.w_hb * fmin(fmax((p.hb_bad - d) * p.hb_inv, 0.0), 1.0);
     return e;
 }
 

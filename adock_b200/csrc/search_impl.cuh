@@ -1189,25 +1189,43 @@ __global__ void __launch_bounds__(256) stage_a_kernel(const __grid_constant__ Se
 }
 
 // ------------------------------------------------------------------------------------------ float64 re-score
-// One warp per state: float64 forward kinematics, exact pairwise inter energy over all receptor atoms (or the
-// grid interpolated in float64 when no receptor atoms are given), out-of-box penalty, intra pairs.
+// One CTA of RS_WARPS warps per state: float64 forward kinematics, exact pairwise inter energy over all receptor atoms
+// (or the grid interpolated in float64 when no receptor atoms are given), out-of-box penalty, intra pairs.
+// Bound by the float64 pair terms (two exponentials each). Receptor atoms outside the pose's bounding box grown by the
+// cutoff are dropped, the rest staged in shared memory; warps take batches of 32 of them, find the pairs inside the
+// cutoff with a float32 distance (widened by its rounding) and queue them, so that the exact distance and the terms run
+// 32 pairs at a time. A warp per pose that tested every receptor atom in float64 for each of its atoms and evaluated
+// the terms wherever one lane was inside took 1,945 us for 8,192 poses x 1,500 receptor atoms, this
+// 407 us.
+#define RS_WARPS 4
+#define RS_LIST 1024   // staged receptor atoms
+
+struct RescoreSmem {   // after the coordinates [3][AM] (double)
+    float4 rec[RS_LIST];               // receptor atoms: xyz, type | flags << 8
+    unsigned short queue[RS_WARPS][64], with[RS_WARPS][64];   // pairs to evaluate: pose atom, staged receptor atom
+    int count[RS_WARPS];
+    float box[6];
+    double inter[RS_WARPS], intra[RS_WARPS];
+};
+
 template <typename GT>
-__global__ void __launch_bounds__(128) rescore64_kernel(const __grid_constant__ SearchParams P, const int* chain_lig, int n,
-                                                        const float* state, double* e_total, double* e_intra,
-                                                        float* Xout, const __grid_constant__ TypeTables ttg,
-                                                        const __grid_constant__ adock_sf_t sf) {
+__global__ void __launch_bounds__(32 * RS_WARPS) rescore64_kernel(const __grid_constant__ SearchParams P, const int* chain_lig,
+                                                                  const float* state, double* e_total, double* e_intra,
+                                                                  float* Xout, const __grid_constant__ TypeTables ttg,
+                                                                  const __grid_constant__ PairPrm64 pp) {
     extern __shared__ double smemd[];
     __shared__ TypeTables tt;
+    __shared__ RescoreSmem S;
     stage_tables(tt, ttg);
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    double* X = smemd + (size_t)wid * P.AM * 3;
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    double *X = smemd, *Y = smemd + P.AM, *Z = smemd + 2 * P.AM;
     const int SDM = 7 + P.KM;
-    const int ch = blockIdx.x * (blockDim.x >> 5) + wid;
-    if (ch >= n) return;
+    const long long ch = blockIdx.x;
     const int l = chain_lig[ch];
     const int4 inf = P.info[l];
     const int na = inf.x, nt = inf.y, np = inf.z, ri = inf.w;
-    const float* s = state + (long long)ch * SDM;
+    const float4* atoms = P.atoms + (long long)l * P.AM;
+    const float* s = state + ch * SDM;
     double qw = s[3], qx = s[4], qy = s[5], qz = s[6];
     const double nq = 1.0 / sqrt(qw * qw + qx * qx + qy * qy + qz * qz);
     qw *= nq; qx *= nq; qy *= nq; qz *= nq;
@@ -1216,9 +1234,13 @@ __global__ void __launch_bounds__(128) rescore64_kernel(const __grid_constant__ 
     const double R20 = 2 * (qx * qz - qy * qw), R21 = 2 * (qy * qz + qx * qw), R22 = 1 - 2 * (qx * qx + qy * qy);
     const float4* tr = P.tors + (long long)l * P.KM * 2;
     double einter = 0.0, eintra = 0.0;
-    const double cut = P.pp.cutoff;
-    for (int a = lane; a < na; a += 32) {
-        const float4 v = P.atoms[(long long)l * P.AM + a];
+    const double cut = pp.cutoff;
+    double* trig = smemd + 3 * P.AM;   // [KM][2] cos, sin
+    float* xf = (float*)(trig + 2 * P.KM);   // [3][AM] float32 coordinates
+    for (int k = tid; k < nt; k += 32 * RS_WARPS) sincos((double)s[7 + k], &trig[2 * k + 1], &trig[2 * k]);
+    __syncthreads();
+    for (int a = tid; a < na; a += 32 * RS_WARPS) {
+        const float4 v = atoms[a];
         double px = v.x, py = v.y, pz = v.z;
         uint32_t m = P.masks[(long long)l * P.AM + a];
         while (m) {
@@ -1226,8 +1248,7 @@ __global__ void __launch_bounds__(128) rescore64_kernel(const __grid_constant__ 
             m &= m - 1;
             if (k >= nt) break;
             const float4 A = tr[2 * k], U = tr[2 * k + 1];
-            double sv, cv;
-            sincos((double)s[7 + k], &sv, &cv);
+            const double cv = trig[2 * k], sv = trig[2 * k + 1];
             const double vx = px - A.x, vy = py - A.y, vz = pz - A.z;
             const double d = U.x * vx + U.y * vy + U.z * vz;
             const double cx = U.y * vz - U.z * vy, cy = U.z * vx - U.x * vz, cz = U.x * vy - U.y * vx;
@@ -1238,27 +1259,13 @@ __global__ void __launch_bounds__(128) rescore64_kernel(const __grid_constant__ 
         const double X0 = R00 * px + R01 * py + R02 * pz + s[0];
         const double X1 = R10 * px + R11 * py + R12 * pz + s[1];
         const double X2 = R20 * px + R21 * py + R22 * pz + s[2];
-        X[3 * a] = X0; X[3 * a + 1] = X1; X[3 * a + 2] = X2;
-        Xout[((long long)ch * P.AM + a) * 3] = (float)X0;
-        Xout[((long long)ch * P.AM + a) * 3 + 1] = (float)X1;
-        Xout[((long long)ch * P.AM + a) * 3 + 2] = (float)X2;
-        const int meta = __float_as_int(v.w);
-        const int ta = (meta >> 16) & 63, slot = meta & 0xffff;
-        double ea = 0.0;
-        if (P.rxyz) {
-            const float* rx = P.rxyz + (long long)ri * P.RN * 3;
-            const int* rt = P.rtyp + (long long)ri * P.RN;
-            const int rn = P.rn[ri];
-            const int fa = tt.flags[ta];
-            for (int b = 0; b < rn; ++b) {
-                const double dx = X0 - rx[3 * b], dy = X1 - rx[3 * b + 1], dz = X2 - rx[3 * b + 2];
-                const double r2 = dx * dx + dy * dy + dz * dz;
-                if (r2 >= cut * cut) continue;
-                const int tb = rt[b] & 63, fb = tt.flags[tb];
-                ea += pair_energy64(sqrt(r2), (double)tt.radius[ta] + (double)tt.radius[tb],
-                                    hyd_pair(fa, fb) | hb_pair(fa, fb), sf.prm);
-            }
-        } else {
+        X[a] = X0; Y[a] = X1; Z[a] = X2;
+        xf[a] = (float)X0; xf[P.AM + a] = (float)X1; xf[2 * P.AM + a] = (float)X2;
+        Xout[(ch * P.AM + a) * 3] = (float)X0;
+        Xout[(ch * P.AM + a) * 3 + 1] = (float)X1;
+        Xout[(ch * P.AM + a) * 3 + 2] = (float)X2;
+        if (!P.rxyz) {
+            const int slot = __float_as_int(v.w) & 0xffff;
             const GT* G = (const GT*)P.flat + P.offs[ri];
             const long long nx = P.dims[3 * ri], ny = P.dims[3 * ri + 1], nz = P.dims[3 * ri + 2];
             const double xx[3] = {X0, X1, X2};
@@ -1272,39 +1279,150 @@ __global__ void __launch_bounds__(128) rescore64_kernel(const __grid_constant__ 
                 fw[d] = fc - (double)i0[d];
             }
             const GT* Gs = G + (long long)slot * nx * ny * nz;
+            double ea = 0.0;
             for (int dx = 0; dx < 2; ++dx)
                 for (int dy = 0; dy < 2; ++dy)
                     for (int dz = 0; dz < 2; ++dz) {
                         const double w = (dx ? fw[0] : 1 - fw[0]) * (dy ? fw[1] : 1 - fw[1]) * (dz ? fw[2] : 1 - fw[2]);
                         ea += w * (double)gload(Gs + ((i0[0] + dx) * ny + (i0[1] + dy)) * nz + (i0[2] + dz));
                     }
+            einter += ea;
         }
         const double xx[3] = {X0, X1, X2};
         for (int d = 0; d < 3; ++d) {
             const double lo = fmax((double)P.lo[3 * ri + d] - xx[d], 0.0), hi = fmax(xx[d] - (double)P.hi[3 * ri + d], 0.0);
-            ea += (double)P.pen * (lo * lo + hi * hi);
+            einter += (double)P.pen * (lo * lo + hi * hi);
         }
-        einter += ea;
     }
-    __syncwarp();
+    __syncthreads();
+    if (P.rxyz) {
+        // bounding box of the pose (everything when a coordinate is not finite)
+        float reach = 0.f;   // largest coordinate: scales the float32 rounding of the distances
+        if (wid == 0) {
+            float lo[3] = {3.4e38f, 3.4e38f, 3.4e38f}, hi[3] = {-3.4e38f, -3.4e38f, -3.4e38f};
+            bool fine = true;
+            for (int a = lane; a < na; a += 32) {
+                const float x[3] = {xf[a], xf[P.AM + a], xf[2 * P.AM + a]};
+                for (int d = 0; d < 3; ++d) {
+                    fine = fine && isfinite(x[d]);
+                    lo[d] = fminf(lo[d], x[d]);
+                    hi[d] = fmaxf(hi[d], x[d]);
+                }
+            }
+            fine = __all_sync(0xffffffffu, fine);
+            for (int d = 0; d < 3; ++d)
+                for (int o = 16; o > 0; o >>= 1) {
+                    lo[d] = fminf(lo[d], __shfl_xor_sync(0xffffffffu, lo[d], o));
+                    hi[d] = fmaxf(hi[d], __shfl_xor_sync(0xffffffffu, hi[d], o));
+                }
+            if (lane == 0)
+                for (int d = 0; d < 3; ++d) {
+                    S.box[d] = fine ? lo[d] : -INFINITY;
+                    S.box[3 + d] = fine ? hi[d] : INFINITY;
+                }
+        }
+        __syncthreads();
+        for (int d = 0; d < 6; ++d) reach = fmaxf(reach, fabsf(S.box[d]));
+        // a float32 distance below the cutoff differs from the exact one by less than 4e-6 of the coordinates
+        const float wide = P.pp.cutoff + 1e-3f + 1e-5f * reach, cut2w = wide * wide;
+        const float lx = S.box[0] - wide, ly = S.box[1] - wide, lz = S.box[2] - wide;
+        const float hx = S.box[3] + wide, hy = S.box[4] + wide, hz = S.box[5] + wide;
+        const float* rx = P.rxyz + (long long)ri * P.RN * 3;
+        const int* rt = P.rtyp + (long long)ri * P.RN;
+        const int rn = P.rn[ri];
+        auto evaluate = [&](int q) {   // queue entry q of this warp
+            const int a = S.queue[wid][q];
+            const float4 B = S.rec[S.with[wid][q]];
+            const double dx = X[a] - B.x, dy = Y[a] - B.y, dz = Z[a] - B.z;
+            const double r2 = dx * dx + dy * dy + dz * dz;
+            if (r2 >= cut * cut) return;
+            const int ta = (__float_as_int(atoms[a].w) >> 16) & 63, fa = tt.flags[ta];
+            const int tb = __float_as_int(B.w) & 63, fb = __float_as_int(B.w) >> 8;
+            einter += pair_energy64(sqrt(r2), (double)tt.radius[ta] + (double)tt.radius[tb], hyd_pair(fa, fb) | hb_pair(fa, fb),
+                                    pp);
+        };
+        int listed = 0;
+        for (int r0 = 0; r0 < rn; r0 += 32 * RS_WARPS) {
+            // stage the next 128 receptor atoms that lie in the box, in receptor order
+            const int r = r0 + tid;
+            bool in = false;
+            float x = 0.f, y = 0.f, z = 0.f;
+            if (r < rn) {
+                x = rx[3 * r]; y = rx[3 * r + 1]; z = rx[3 * r + 2];
+                in = !(x < lx || x > hx || y < ly || y > hy || z < lz || z > hz);
+            }
+            const unsigned bal = __ballot_sync(0xffffffffu, in);
+            if (lane == 0) S.count[wid] = __popc(bal);
+            __syncthreads();
+            int at = listed + __popc(bal & ((1u << lane) - 1u));
+            for (int w = 0; w < RS_WARPS; ++w) {
+                if (w < wid) at += S.count[w];
+                listed += S.count[w];
+            }
+            if (in) {
+                const int tb = rt[r] & 63;   // index kept inside the 64-entry type tables
+                S.rec[at] = make_float4(x, y, z, __int_as_float(tb | (tt.flags[tb] << 8)));
+            }
+            __syncthreads();
+            if (listed + 32 * RS_WARPS <= RS_LIST && r0 + 32 * RS_WARPS < rn) continue;
+            // batches of 32 staged atoms per warp against every atom of the pose
+            int queued = 0;
+            for (int b0 = 32 * wid; b0 < listed; b0 += 32 * RS_WARPS) {
+                const int bi = b0 + lane;
+                const bool have = bi < listed;
+                const float4 B = S.rec[have ? bi : 0];
+                for (int a = 0; a < na; ++a) {
+                    const float dx = xf[a] - B.x, dy = xf[P.AM + a] - B.y, dz = xf[2 * P.AM + a] - B.z;
+                    const bool near = have && !(dx * dx + dy * dy + dz * dz > cut2w);
+                    const unsigned m = __ballot_sync(0xffffffffu, near);
+                    if (near) {
+                        const int q = queued + __popc(m & ((1u << lane) - 1u));
+                        S.queue[wid][q] = (unsigned short)a;
+                        S.with[wid][q] = (unsigned short)bi;
+                    }
+                    queued += __popc(m);
+                    if (queued >= 32) {   // at most 63 queued: evaluate the last 32
+                        __syncwarp();
+                        queued -= 32;
+                        evaluate(queued + lane);
+                        __syncwarp();
+                    }
+                }
+            }
+            __syncwarp();
+            if (lane < queued) evaluate(lane);
+            listed = 0;
+            __syncthreads();
+        }
+    }
     const int2* pairs = P.pairs + (long long)l * P.P_pad;
     const int nslot = ((np + 31) >> 5) << 5;
-    for (int q = lane; q < nslot; q += 32) {
+    for (int q = tid; q < nslot; q += 32 * RS_WARPS) {
         const int2 pr = pairs[q];
         if (pr.x < 0) continue;
         const int i = pr.x & 0xff, j = (pr.x >> 8) & 0xff, fl = pr.x >> 16;
-        const double dx = X[3 * i] - X[3 * j], dy = X[3 * i + 1] - X[3 * j + 1], dz = X[3 * i + 2] - X[3 * j + 2];
+        const double dx = X[i] - X[j], dy = Y[i] - Y[j], dz = Z[i] - Z[j];
         const double r = sqrt(dx * dx + dy * dy + dz * dz);
         if (r >= cut) continue;
-        const int ti = (__float_as_int(P.atoms[(long long)l * P.AM + i].w) >> 16) & 63;
-        const int tj = (__float_as_int(P.atoms[(long long)l * P.AM + j].w) >> 16) & 63;
-        eintra += pair_energy64(r, (double)tt.radius[ti] + (double)tt.radius[tj], fl, sf.prm);
+        const int ti = (__float_as_int(atoms[i].w) >> 16) & 63;
+        const int tj = (__float_as_int(atoms[j].w) >> 16) & 63;
+        eintra += pair_energy64(r, (double)tt.radius[ti] + (double)tt.radius[tj], fl, pp);
     }
     einter = warp_sum_d(einter);
     eintra = warp_sum_d(eintra);
     if (lane == 0) {
-        e_total[ch] = einter + eintra;
-        e_intra[ch] = eintra;
+        S.inter[wid] = einter;
+        S.intra[wid] = eintra;
+    }
+    __syncthreads();
+    if (tid == 0) {
+        double ei = 0.0, ea = 0.0;
+        for (int w = 0; w < RS_WARPS; ++w) {
+            ei += S.inter[w];
+            ea += S.intra[w];
+        }
+        e_total[ch] = ei + ea;
+        e_intra[ch] = ea;
     }
 }
 
@@ -1410,10 +1528,8 @@ int launch_stage_a(const SearchParams& P, long long blocks, const float* conf, i
 template <typename GT>
 int launch_rescore64(const SearchParams& P, const int* cl, int n, const float* state, double* et, double* ei, float* X,
                      const TypeTables& tt, const adock_sf_t& sf, cudaStream_t st) {
-    const int wpb = 4;
-    const size_t smem = (size_t)wpb * P.AM * 3 * sizeof(double);
-    const unsigned blocks = (unsigned)((n + wpb - 1) / wpb);
-    rescore64_kernel<GT><<<blocks, 32 * wpb, smem, st>>>(P, cl, n, state, et, ei, X, tt, sf);
+    const size_t smem = (3 * (size_t)P.AM + 2 * (size_t)P.KM) * sizeof(double) + 3 * (size_t)P.AM * sizeof(float);
+    rescore64_kernel<GT><<<n, 32 * RS_WARPS, smem, st>>>(P, cl, state, et, ei, X, tt, make_pair_prm64(sf.prm));
     ADOCK_CUDA(cudaGetLastError());
     return ADOCK_OK;
 }
