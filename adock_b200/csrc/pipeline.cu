@@ -19,11 +19,41 @@ static inline int pow2_at_least(int x) {
 
 // ------------------------------------------------------------------------------------------ block primitives
 // Ascending bitonic sort of (key, index) pairs in shared memory; n is a power of two; ties break on the index, so
-// the order is the stable order of the keys.
+// the order is the stable order of the keys. A warp keeps the compare-exchanges of distance below 32 of its 32-element
+// runs in registers (shuffles, no block barrier): 28 of the 78 stages of 4,096 elements stay in shared memory
+// (64 ligands x 3,072 totals: 54 -> 48 us).
+template <typename K>
+__device__ __forceinline__ void sort_exchange(K& a, int& ia, K b, int ib, bool keep_low) {
+    const bool greater = (a > b) || (a == b && ia > ib);   // the pair is (a, b) with a this lane's
+    if (greater == keep_low) { a = b; ia = ib; }
+}
+
 template <typename K>
 __device__ void block_sort_pairs(K* key, int* idx, int n) {
-    for (int k = 2; k <= n; k <<= 1) {
-        for (int j = k >> 1; j > 0; j >>= 1) {
+    const int lane = threadIdx.x & 31;
+    auto runs = [&](int k, int j0) {   // distances j0, j0 / 2, .., 1 (j0 < 32) of step k
+        for (int base = threadIdx.x - lane; base < n; base += blockDim.x) {
+            const int i = base + lane;
+            const bool have = i < n;
+            K a = have ? key[i] : K(0);
+            int ia = have ? idx[i] : 0;
+            for (int kk = j0 ? k : 2; kk <= k; kk <<= 1)
+                for (int j = j0 ? j0 : kk >> 1; j > 0; j >>= 1) {
+                    const K b = __shfl_xor_sync(0xffffffffu, a, j);
+                    const int ib = __shfl_xor_sync(0xffffffffu, ia, j);
+                    const bool up = (i & kk) == 0, low = (i & j) == 0;
+                    sort_exchange(a, ia, b, ib, up == low);
+                }
+            if (have) {
+                key[i] = a;
+                idx[i] = ia;
+            }
+        }
+        __syncthreads();
+    };
+    runs(min(n, 32), 0);   // steps 2 .. 32
+    for (int k = 64; k <= n; k <<= 1) {
+        for (int j = k >> 1; j >= 32; j >>= 1) {
             for (int i = threadIdx.x; i < n; i += blockDim.x) {
                 const int p = i ^ j;
                 if (p > i) {
@@ -39,6 +69,7 @@ __device__ void block_sort_pairs(K* key, int* idx, int n) {
             }
             __syncthreads();
         }
+        runs(k, 16);
     }
 }
 
@@ -68,13 +99,13 @@ __device__ int block_exclusive_scan(int flag, int* warp_tot, int* total) {
 }
 
 // ------------------------------------------------------------------------------------------ conformers
-// Ligand-frame heavy-atom coordinates of torsion set `trial` of ligand l (radii rad [AM]) into X ([3][AM] in shared
-// memory) and
+// Ligand-frame heavy-atom coordinates of torsion set `trial` of ligand l (radii rad [AM], torsion axes tr [KM][2] in
+// shared memory) into X ([3][AM] in shared memory) and
 // the set's torsion angles into th (shared, KM); returns the intra-ligand energy (all lanes). Set 0 is the input
 // conformer (all angles 0); the others draw each torsion angle uniformly in [-pi, pi) from the counter-based
 // stream (seed, ligand, set, torsion).
 __device__ float conformer_set(const SearchParams& P, int l, int trial, unsigned long long seed, const float* rad,
-                               float* X, float* th, float* cs, float* sn, int lane) {
+                               const float4* tr, float* X, float* th, float* cs, float* sn, int lane) {
     const int4 inf = P.info[l];
     const int na = inf.x, nt = inf.y, np = inf.z;
     const int AM = P.AM;
@@ -87,7 +118,6 @@ __device__ float conformer_set(const SearchParams& P, int l, int trial, unsigned
         sn[k] = sv;
     }
     __syncwarp();
-    const float4* tr = P.tors + (long long)l * P.KM * 2;
     for (int a = lane; a < AM; a += 32) {
         float px = 0.f, py = 0.f, pz = 0.f;
         if (a < na) {
@@ -113,15 +143,14 @@ __device__ float conformer_set(const SearchParams& P, int l, int trial, unsigned
     float e = 0.f;
     const int2* pr = P.pairs + (long long)l * P.P_pad;
     const int nslot = pad32i(np);
-    for (int q = lane; q < nslot; q += 32) {
+#pragma unroll 4
+    for (int q = lane; q < nslot; q += 32) {   // branch-free: four pairs in flight
         const int2 rec = pr[q];
-        if (rec.x < 0) continue;
-        const int i = rec.x & 0xff, j = (rec.x >> 8) & 0xff, fl = rec.x >> 16;
+        const int x = rec.x < 0 ? 0 : rec.x, i = x & 0xff, j = (x >> 8) & 0xff, fl = x >> 16;
         const float rx = X[i] - X[j], ry = X[AM + i] - X[AM + j], rz = X[2 * AM + i] - X[2 * AM + j];
         const float r = sqrtf(rx * rx + ry * ry + rz * rz);
-        if (r >= P.pp.cutoff) continue;
-        float de;
-        e += pair_energy(r, rad[i] + rad[j], fl, P.pp, de);
+        const float ep = pair_energy(r, rad[i] + rad[j], fl, P.pp);
+        e += rec.x < 0 || r >= P.pp.cutoff ? 0.f : ep;
     }
     e = warp_sum(e);
     __syncwarp();
@@ -131,7 +160,7 @@ __device__ float conformer_set(const SearchParams& P, int l, int trial, unsigned
 // One CTA per ligand: the intra energy of NT torsion sets, then the C lowest (ties: lower set index) in ascending
 // energy order, written as angles theta [L, C, KM], heavy-atom coordinates conf [L, C, AM, 3] (0 past na) and
 // energies e [L, C].
-__global__ void __launch_bounds__(256) conformer_kernel(const __grid_constant__ SearchParams P, int NT, int C,
+__global__ void __launch_bounds__(1024) conformer_kernel(const __grid_constant__ SearchParams P, int NT, int C,
                                                         unsigned long long seed, float* theta_out, float* conf_out,
                                                         float* e_out, const __grid_constant__ TypeTables tt) {
     extern __shared__ float csm[];
@@ -142,6 +171,7 @@ __global__ void __launch_bounds__(256) conformer_kernel(const __grid_constant__ 
     int* sel = (int*)(csm + NT);                // [C]
     float* rad = csm + NT + C;                  // [AM]
     float* ws = rad + AM + wid * (3 * AM + 3 * KM);
+    __shared__ float4 tr[2 * 32];               // torsion axes (KM <= 32)
     float* X = ws;
     float* th = ws + 3 * AM;
     float* cs = th + KM;
@@ -150,9 +180,10 @@ __global__ void __launch_bounds__(256) conformer_kernel(const __grid_constant__ 
         const int typ = __float_as_int(P.atoms[(long long)l * AM + a].w) >> 16;
         rad[a] = tt.radius[typ < 0 ? 0 : typ & 63];
     }
+    for (int k = threadIdx.x; k < 2 * KM; k += blockDim.x) tr[k] = P.tors[(long long)l * KM * 2 + k];
     __syncthreads();
     for (int t = wid; t < NT; t += nw) {
-        const float e = conformer_set(P, l, t, seed, rad, X, th, cs, sn, lane);
+        const float e = conformer_set(P, l, t, seed, rad, tr, X, th, cs, sn, lane);
         if (lane == 0) e_s[t] = (e == e) ? e : 3.4e38f;   // a NaN energy ranks last
     }
     __syncthreads();
@@ -168,7 +199,7 @@ __global__ void __launch_bounds__(256) conformer_kernel(const __grid_constant__ 
     __syncthreads();
     for (int r = wid; r < C; r += nw) {
         const int t = sel[r];
-        conformer_set(P, l, t, seed, rad, X, th, cs, sn, lane);
+        conformer_set(P, l, t, seed, rad, tr, X, th, cs, sn, lane);
         const long long o = (long long)l * C + r;
         for (int k = lane; k < KM; k += 32) theta_out[o * KM + k] = th[k];
         for (int a = lane; a < AM; a += 32) {
@@ -427,7 +458,9 @@ extern "C" int adock_conformers(const adock_ligands_t* lig, const adock_work_t* 
     ADOCK_CHECK_ARG(NT >= 1 && NT <= 4096, "NT must be in [1, 4096] (got %d)", NT);
     ADOCK_CHECK_ARG(C >= 1 && C <= NT, "C must be in [1, NT] (got %d)", C);
     ADOCK_CHECK_ARG(theta && conf && e, "null array argument");
-    const int threads = 256;
+    // a warp per torsion set: one CTA per ligand, so few ligands need many warps (64 ligands x 64 sets: 135 us with 8
+    // warps, 73 us with 32)
+    const int threads = 32 * min(32, max(8, NT / 2));
     const size_t smem = ((size_t)NT + C + P.AM + (threads / 32) * (3 * (size_t)P.AM + 3 * (size_t)P.KM)) * sizeof(float);
     ADOCK_CUDA(cudaFuncSetAttribute(conformer_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     conformer_kernel<<<lig->L, threads, smem, (cudaStream_t)stream>>>(P, NT, C, splitmix(seed ^ 0xC0F0A11CE5ULL), theta,
