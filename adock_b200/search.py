@@ -56,10 +56,18 @@ def _boxes(prob, boxes_c, boxes_s, step):
     [B, 3], and the box of each ligand [L]."""
     L = prob.lb.L
     c = _host(boxes_c).reshape(L, 3)
-    s = np.stack([_host(x) for x in boxes_s]).reshape(L, 3) if len(boxes_s) == L else np.tile(_host(boxes_s), (L, 1))
+    if len(boxes_s) != L:
+        s = np.tile(_host(boxes_s), (L, 1))
+    elif torch.is_tensor(boxes_s) or any(torch.is_tensor(x) for x in boxes_s):
+        s = np.stack([_host(x) for x in boxes_s]).reshape(L, 3)
+    else:
+        s = np.array(boxes_s, np.float64).reshape(L, 3)
     rec = _host(prob.rec_idx, np.int64).reshape(L)
     key = np.concatenate([rec[:, None].astype(np.float64), np.round(c, 6), np.round(s, 6)], 1)
-    uniq, first, lig_box = np.unique(key, axis=0, return_index=True, return_inverse=True)
+    if (key == key[0]).all():   # one pocket, the usual screen: no sort of the rows
+        first, lig_box = np.zeros(1, np.int64), np.zeros(L, np.int64)
+    else:
+        _, first, lig_box = np.unique(key, axis=0, return_index=True, return_inverse=True)
     table = np.concatenate([c[first], s[first]], 1).astype(np.float32)
     # points per axis of arange(-s/2 + 1, s/2 - 1 + 1e-6, step)
     n = np.array([[len(np.arange(-sd / 2 + 1.0, sd / 2 - 1.0 + 1e-6, step)) for sd in row] for row in s[first]],
@@ -74,6 +82,18 @@ def _quaternions(Q, seed):
     return (q / np.linalg.norm(q, axis=1, keepdims=True)).astype(np.float32)
 
 
+def _upload(arrays, dev):
+    """Device copies of small 32-bit host arrays through one transfer (a transfer each costs about 15 us of host time)."""
+    flat = torch.as_tensor(np.concatenate([np.ascontiguousarray(a).reshape(-1).view(np.int32) for a in arrays.values()]),
+                           device=dev)
+    out, at = {}, 0
+    for k, a in arrays.items():
+        t = flat[at:at + a.size]
+        out[k] = (t.view(torch.float32) if a.dtype == np.float32 else t).view(a.shape)
+        at += a.size
+    return out
+
+
 @torch.no_grad()
 def stage_a_starts(prob, kp, boxes_c, boxes_s, cfg, seed):
     """Stage A on the device: start states [L * M, 7 + KM] (ligand-major) and their Stage-A energies [L * M]."""
@@ -83,15 +103,15 @@ def stage_a_starts(prob, kp, boxes_c, boxes_s, cfg, seed):
     C = min(cfg["stageA_conformers"], NT)
     Q = cfg["stageA_rotations"]
     step = cfg["stageA_translation_step"]
-    table, box_rec, box_n, lig_box = _boxes(prob, boxes_c, boxes_s, step)
+    quats = _quaternions(Q, seed)
     slot = prob.gs.slot.cpu().numpy() if torch.is_tensor(prob.gs.slot) else np.asarray(prob.gs.slot)
+    table, box_rec, box_n, lig_box = _boxes(prob, boxes_c, boxes_s, step)
     box_slot = slot[box_rec, 0].astype(np.int32)          # type 0 (C_H) is the probe, as in the reference
     assert (box_slot >= 0).all(), "the probe type (C_H) has no map"
     nt_max = int(box_n.prod(1).max())
-    host = {"table": table, "box_rec": box_rec, "box_slot": box_slot, "box_n": box_n, "lig_box": lig_box,
-            "quats": _quaternions(Q, seed)}
-    d = {k: torch.as_tensor(v, device=dev) for k, v in host.items()}
-    theta, conf, e_conf = kp.conformers(NT, C, seed)
+    theta, conf, e_conf = kp.conformers(NT, C, seed)      # runs while the tables are uploaded
+    d = _upload({"table": table, "box_rec": box_rec, "box_slot": box_slot, "box_n": box_n, "lig_box": lig_box,
+                 "quats": quats}, dev)
     trans, ntrans = kp.lattice(len(table), d["table"], d["box_rec"], d["box_slot"], d["box_n"], step,
                                cfg.get("stageA_probe_max", 0.0), nt_max)
     best_e, best_i = kp.stage_a_boxes(conf, d["quats"], trans, ntrans, d["lig_box"], cfg.get("stageA_atom_cap", 1e9))
