@@ -223,7 +223,7 @@ struct Distances {
 
 // Vina maps. Bound by instruction issue and the two exponentials per (atom, point, radius). A thread per point that
 // added five sums per ligand type and tested every staged atom took 687 us for 8,000 receptor atoms, 81^3 points and 8
-// types (4 radii), this 272-295 us.
+// types (4 radii), this 295 us.
 // PER_TERM writes the five unweighted terms: the first two sums then hold one of the first three per sweep.
 template <int PP, bool PER_TERM>
 __global__ void __launch_bounds__(Tile<PP>::THREADS, PP == 2 ? 3 : 8) grid_vina_kernel(const float* __restrict__ rxyz,

@@ -123,8 +123,8 @@ struct WSLayout {
         const int DM = 6 + KM, SD = 7 + KM;
         int o = 0;
         X = o; o += 4 * AM;    // world coordinates and radii, [4][AM] (x, y, z, radius arrays)
-        FT = o; o += 8 * AM;   // forces of the pair loop, [3][AM]; then float4 (force, torsion bitmask) and float4
-                               // (torque, 0) per atom
+        FT = o; o += 8 * AM;   // forces [3][AM] (and the exact energy [AM]); then float4 (force, torsion bitmask) and
+                               // float4 (torque, 0) per atom
         RT = o; o += exact ? 4 * EX_TILE : 0;   // a tile of receptor atoms, float4 (xyz, type | flags << 8)
         V = o; o += 4 * DM;    // BFGS vectors, float4 (p, -H y, y, g) per component
         ap = o; o += 4 * KM;
@@ -162,16 +162,13 @@ struct Chain {
     int rn;
     const int* nb;
     int nbn;
-    int exact;
-    float3 ref[APL];
-    int slot[APL];
-    int typ[APL];
-    uint32_t mask[APL];
+    const float4* atoms;     // this ligand's rows of the working layout
+    const uint32_t* masks;
 };
 
 template <int APL, typename GT>
 __device__ __forceinline__ void load_chain(Chain<APL>& c, const SearchParams& P, const TypeTables& tt, int l, float* ws,
-                                           const WSLayout& L, int lane, int exact, const int* nb, int nbn) {
+                                           const WSLayout& L, int lane, const int* nb, int nbn) {
     const int4 inf = P.info[l];
     c.na = inf.x; c.nt = inf.y; c.np = inf.z;
     c.nrounds = (inf.z + 31) >> 5;
@@ -186,23 +183,16 @@ __device__ __forceinline__ void load_chain(Chain<APL>& c, const SearchParams& P,
         c.o[d] = P.origin[3 * ri + d]; c.lo[d] = P.lo[3 * ri + d]; c.hi[d] = P.hi[3 * ri + d];
     }
     c.fmx[0] = (float)(nx - 1) - 1e-4f; c.fmx[1] = (float)(ny - 1) - 1e-4f; c.fmx[2] = (float)(nz - 1) - 1e-4f;
-    c.exact = exact;
     c.rx = P.rxyz ? P.rxyz + (long long)ri * P.RN * 3 : nullptr;
     c.rt = P.rtyp ? P.rtyp + (long long)ri * P.RN : nullptr;
     c.rn = P.rn ? P.rn[ri] : 0;
     c.nb = nb; c.nbn = nbn;
-    const float4* at = P.atoms + (long long)l * P.AM;
-    const uint32_t* mk = P.masks + (long long)l * P.AM;
-#pragma unroll
-    for (int i = 0; i < APL; ++i) {
-        const int a = lane + 32 * i;
-        const float4 v = at[a];
-        c.ref[i] = make_float3(v.x, v.y, v.z);
-        const int meta = __float_as_int(v.w);
-        c.slot[i] = meta & 0xffff;
-        c.typ[i] = meta >> 16;
-        c.mask[i] = mk[a];
-        ws[L.X + 3 * 32 * APL + a] = tt.radius[c.typ[i] < 0 ? 0 : c.typ[i] & 63];
+    c.atoms = P.atoms + (long long)l * P.AM;
+    c.masks = P.masks + (long long)l * P.AM;
+#pragma unroll 1
+    for (int a = lane; a < 32 * APL; a += 32) {
+        const int typ = __float_as_int(c.atoms[a].w) >> 16;
+        ws[L.X + 3 * 32 * APL + a] = tt.radius[typ < 0 ? 0 : typ & 63];
     }
     const float4* tr = P.tors + (long long)l * P.KM * 2;
     float4* ap = (float4*)(ws + L.ap);
@@ -309,27 +299,19 @@ __device__ __forceinline__ void push_forces(int w, int repeats, float3 f, float*
     __syncwarp();
 }
 
-// Intra-ligand pairs: adds the lane's slots to its share e of the energy (returned) and, with GRAD, the forces on the
-// lane's atoms (lane + 32 i) to F. An atom's contributions are added in the order round, first atoms before second atoms, lane.
+// Intra-ligand pairs: adds the lane's slots to its share e of the energy (returned) and, with GRAD, the forces to the
+// atoms' entries of [3][AM] in shared memory. An atom's contributions are added in the order round, first atoms before second atoms, lane.
 // Bound by instruction issue and the latency of the rounds' shared-memory updates (about 95 instructions per slot for
 // the pair term, 66 per round for the two sides). With shared float atomics for the forces and the pair parameters read
 // through a generic pointer this loop took 10.3 k of a single warp's 19 k cycles per evaluation (24 atoms, 7 rounds);
 // now 2.9 k (averaged over evaluations with and without the gradient). Summing in registers instead was slower: owners pulling by shuffles (132 instructions per round), or
 // per-atom slot lists over forces left in shared memory (12 wavefronts per entry from bank conflicts).
 template <int APL, bool GRAD>
-__device__ __forceinline__ float pair_terms(float* ws, const WSLayout& L, const Chain<APL>& c, const PairPrm& pp,
-                                            float3 (&F)[APL], float e, int lane) {
+__device__ __forceinline__ float pair_terms(float* ws, const WSLayout& L, const Chain<APL>& c, const PairPrm& pp, float e,
+                                            int lane) {
     constexpr int AM = 32 * APL;
     const float* X = ws + L.X;
     float* FF = ws + L.FT;
-    if (GRAD) {
-#pragma unroll
-        for (int i = 0; i < APL; ++i) {
-            const int a = lane + 32 * i;
-            FF[a] = F[i].x; FF[AM + a] = F[i].y; FF[2 * AM + a] = F[i].z;
-        }
-    }
-    __syncwarp();
     // two rounds in flight; the next two rounds' records are loaded while these are evaluated
     const int empty = lane * (33 << PR_NEXT);   // atom 0 twice, linked to itself, first of nothing
     const int2 none = make_int2(-1, 0);
@@ -354,19 +336,11 @@ __device__ __forceinline__ float pair_terms(float* ws, const WSLayout& L, const 
         pa = qa;
         pb = qb;
     }
-    if (GRAD) {
-#pragma unroll
-        for (int i = 0; i < APL; ++i) {
-            const int a = lane + 32 * i;
-            F[i] = make_float3(FF[a], FF[AM + a], FF[2 * AM + a]);
-        }
-    }
-    __syncwarp();
     return e;
 }
 
 // Exact inter energy of the lane's atoms (positions in shared memory) with the receptor atoms, or the chain's
-// neighbour list: sums in list order, and with `grad` the forces into F. A tile of receptor atoms is staged in shared
+// neighbour list, into inter [AM], and the forces, into [3][AM], summed in list order. A tile of receptor atoms is staged in shared
 // memory; each lane first collects the tile's atoms inside the cutoff of its atom as a bit mask (a few instructions per
 // pair, no branches), then evaluates the pair terms of its set bits, two in flight, so that the terms run with most
 // lanes busy: some 50 of a pose's 300 neighbours are inside the 8 A cutoff of one atom. Bound by instruction issue.
@@ -374,8 +348,7 @@ __device__ __forceinline__ float pair_terms(float* ws, const WSLayout& L, const 
 // per evaluation (300 neighbours, 14 warps per SM), this about 31 k.
 template <int APL>
 __device__ __forceinline__ void exact_terms(float* ws, const WSLayout& L, const Chain<APL>& c, const SearchParams& P,
-                                            const TypeTables& tt, float (&inter)[APL], float3 (&F)[APL], int lane,
-                                            bool grad) {
+                                            const TypeTables& tt, int lane) {
     constexpr int AM = 32 * APL;
     const float* X = ws + L.X;
     float4* RT = (float4*)(ws + L.RT);
@@ -387,8 +360,10 @@ __device__ __forceinline__ void exact_terms(float* ws, const WSLayout& L, const 
         const int tb = c.rt[b] & 63;   // index kept inside the 64-entry type tables
         return make_float4(c.rx[3 * b], c.rx[3 * b + 1], c.rx[3 * b + 2], __int_as_float(tb | (tt.flags[tb] << 8)));
     };
+    float* FF = ws + L.FT;
+    float* inter = FF + 3 * AM;
 #pragma unroll
-    for (int i = 0; i < APL; ++i) inter[i] = 0.f;
+    for (int i = 0; i < 4 * APL; ++i) FF[lane + 32 * i] = 0.f;
     float4 n0 = fetch(lane), n1 = fetch(32 + lane);
 #pragma unroll 1
     for (int t0 = 0; t0 < n; t0 += EX_TILE) {
@@ -399,10 +374,8 @@ __device__ __forceinline__ void exact_terms(float* ws, const WSLayout& L, const 
         n0 = fetch(t0 + EX_TILE + lane);
         n1 = fetch(t0 + EX_TILE + 32 + lane);
         const unsigned long long valid = n - t0 >= 64 ? ~0ull : (1ull << (n - t0)) - 1ull;
-#pragma unroll
-        for (int i = 0; i < APL; ++i) {
-            if (32 * i >= c.na) break;
-            const int a = lane + 32 * i;
+#pragma unroll 1
+        for (int a = lane; a - lane < c.na; a += 32) {
             const float X0 = X[a], X1 = X[AM + a], X2 = X[2 * AM + a];
             unsigned m0 = 0, m1 = 0;
 #pragma unroll 8
@@ -416,11 +389,11 @@ __device__ __forceinline__ void exact_terms(float* ws, const WSLayout& L, const 
                 m1 |= (r2 >= cut2 ? 0u : 1u) << b;
             }
             unsigned long long m = a < c.na ? (((unsigned long long)m1 << 32) | m0) & valid : 0ull;
-            const int ta = c.typ[i] & 63;
+            const int ta = (__float_as_int(c.atoms[a].w) >> 16) & 63;
             const float ra = tt.radius[ta];
             const int fa = tt.flags[ta];
-            float ea = inter[i];
-            float3 f = F[i];
+            float ea = inter[a];
+            float3 f = make_float3(FF[a], FF[AM + a], FF[2 * AM + a]);
             const int most = __reduce_max_sync(0xffffffffu, __popcll(m));
 #pragma unroll 1
             for (int t = 0; t < most; t += 2) {
@@ -443,8 +416,8 @@ __device__ __forceinline__ void exact_terms(float* ws, const WSLayout& L, const 
                     }
                 }
             }
-            inter[i] = ea;
-            F[i] = f;
+            inter[a] = ea;
+            FF[a] = f.x; FF[AM + a] = f.y; FF[2 * AM + a] = f.z;
         }
     }
 }
@@ -477,6 +450,7 @@ __device__ __forceinline__ float eval_eg(float* ws, const WSLayout& L, const flo
     const float R00 = 1 - 2 * (qy * qy + qz * qz), R01 = 2 * (qx * qy - qz * qw), R02 = 2 * (qx * qz + qy * qw);
     const float R10 = 2 * (qx * qy + qz * qw), R11 = 1 - 2 * (qx * qx + qz * qz), R12 = 2 * (qy * qz - qx * qw);
     const float R20 = 2 * (qx * qz - qy * qw), R21 = 2 * (qy * qz + qx * qw), R22 = 1 - 2 * (qx * qx + qy * qy);
+#pragma unroll 1
     for (int k = lane; k < c.nt; k += 32) {
         float sv, cv;
         __sincosf(s[7 + k], &sv, &cv);
@@ -485,69 +459,70 @@ __device__ __forceinline__ float eval_eg(float* ws, const WSLayout& L, const flo
     }
     __syncwarp();
     float e = 0.f;
-    float3 F[APL];   // dE/dX of the lane's atoms
-    float inter[APL];
+    float* FF = ws + L.FT;   // forces dE/dX, [3][AM]
     const GT* grid = (const GT*)c.grid;
-#pragma unroll
-    for (int i = 0; i < APL; ++i) {
-        const int a = lane + 32 * i;
-        F[i] = make_float3(0.f, 0.f, 0.f);
-        if (a < c.na) {
-            float px = c.ref[i].x, py = c.ref[i].y, pz = c.ref[i].z;
-            uint32_t m = c.mask[i];
-            while (m) {
-                const int k = __ffs(m) - 1;
-                m &= m - 1;
-                const float4 A = ap[k], U = au[k];
-                const float cv = cs[k], sv = sn[k];
-                const float vx = px - A.x, vy = py - A.y, vz = pz - A.z;
-                const float d = U.x * vx + U.y * vy + U.z * vz;
-                const float cx = U.y * vz - U.z * vy, cy = U.z * vx - U.x * vz, cz = U.x * vy - U.y * vx;
-                px = A.x + vx * cv + cx * sv + U.x * d * (1 - cv);
-                py = A.y + vy * cv + cy * sv + U.y * d * (1 - cv);
-                pz = A.z + vz * cv + cz * sv + U.z * d * (1 - cv);
-            }
-            const float X0 = R00 * px + R01 * py + R02 * pz + t0;
-            const float X1 = R10 * px + R11 * py + R12 * pz + t1;
-            const float X2 = R20 * px + R21 * py + R22 * pz + t2;
-            X[a] = X0;
-            X[AM + a] = X1;
-            X[2 * AM + a] = X2;
+    // The lane's atoms; rolled, and the ligand rows read again each time: the loop saves code, and instruction-cache misses
+    // were the kernel's largest stall (1.95 of 6.9 cycles per issue). With the other rolled loops and the one line-search
+    // step: 256 ligands x 32 chains, start + 8 steps 17.6 -> 14.0 ms.
+    auto place = [&](int a, float4 v) {
+        float px = v.x, py = v.y, pz = v.z;
+        uint32_t m = c.masks[a];
+        while (m) {
+            const int k = __ffs(m) - 1;
+            m &= m - 1;
+            const float4 A = ap[k], U = au[k];
+            const float cv = cs[k], sv = sn[k];
+            const float vx = px - A.x, vy = py - A.y, vz = pz - A.z;
+            const float d = U.x * vx + U.y * vy + U.z * vz;
+            const float cx = U.y * vz - U.z * vy, cy = U.z * vx - U.x * vz, cz = U.x * vy - U.y * vx;
+            px = A.x + vx * cv + cx * sv + U.x * d * (1 - cv);
+            py = A.y + vy * cv + cy * sv + U.y * d * (1 - cv);
+            pz = A.z + vz * cv + cz * sv + U.z * d * (1 - cv);
         }
+        // spelled out: poses round the same whatever code surrounds them
+        X[a] = __fmaf_rn(R02, pz, __fmaf_rn(R00, px, __fmul_rn(R01, py))) + t0;
+        X[AM + a] = __fmaf_rn(R12, pz, __fmaf_rn(R10, px, __fmul_rn(R11, py))) + t1;
+        X[2 * AM + a] = __fmaf_rn(R22, pz, __fmaf_rn(R20, px, __fmul_rn(R21, py))) + t2;
+    };
+    if constexpr (EX) {
+#pragma unroll 1
+        for (int a = lane; a < c.na; a += 32) place(a, c.atoms[a]);
+        __syncwarp();
+        exact_terms<APL>(ws, L, c, P, tt, lane);
     }
-    if constexpr (EX) exact_terms<APL>(ws, L, c, P, tt, inter, F, lane, grad);
-#pragma unroll
-    for (int i = 0; i < APL; ++i) {
-        const int a = lane + 32 * i;
-        if (a < c.na) {
-            const float X0 = X[a], X1 = X[AM + a], X2 = X[2 * AM + a];
-            float ea, gg[3];
-            if constexpr (EX) {
-                ea = inter[i];
-                gg[0] = F[i].x; gg[1] = F[i].y; gg[2] = F[i].z;
-            } else {
-                ea = trilinear<GT>(grid + (long long)c.slot[i] * c.n3, c.ny, c.nz, c.o, c.fmx, P.inv_s, X0, X1, X2,
-                                   gg[0], gg[1], gg[2]);
-            }
-            const float xx[3] = {X0, X1, X2};
-#pragma unroll
-            for (int d = 0; d < 3; ++d) {
-                const float lo = fmaxf(c.lo[d] - xx[d], 0.f), hi = fmaxf(xx[d] - c.hi[d], 0.f);
-                ea += P.pen * (lo * lo + hi * hi);
-                gg[d] += P.pen * (-2.f * lo + 2.f * hi);
-            }
-            e += ea;
-            F[i] = make_float3(gg[0], gg[1], gg[2]);
+#pragma unroll 1
+    for (int a = lane; a < c.na; a += 32) {
+        float ea, gg[3];
+        if constexpr (EX) {
+            ea = FF[3 * AM + a];
+            gg[0] = FF[a]; gg[1] = FF[AM + a]; gg[2] = FF[2 * AM + a];
+        } else {
+            const float4 v = c.atoms[a];
+            place(a, v);
+            ea = trilinear<GT>(grid + (long long)(__float_as_int(v.w) & 0xffff) * c.n3, c.ny, c.nz, c.o, c.fmx, P.inv_s, X[a],
+                               X[AM + a], X[2 * AM + a], gg[0], gg[1], gg[2]);
         }
+        const float xx[3] = {X[a], X[AM + a], X[2 * AM + a]};
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            const float lo = fmaxf(c.lo[d] - xx[d], 0.f), hi = fmaxf(xx[d] - c.hi[d], 0.f);
+            ea += P.pen * (lo * lo + hi * hi);
+            gg[d] += P.pen * (-2.f * lo + 2.f * hi);
+        }
+        e += ea;
+        FF[a] = gg[0];
+        FF[AM + a] = gg[1];
+        FF[2 * AM + a] = gg[2];
     }
     __syncwarp();
     if (!grad) {
-        e = warp_sum(pair_terms<APL, false>(ws, L, c, P.pp, F, e, lane));
+        e = warp_sum(pair_terms<APL, false>(ws, L, c, P.pp, e, lane));
         __syncwarp();
         return e;
     }
-    e = pair_terms<APL, true>(ws, L, c, P.pp, F, e, lane);
+    e = pair_terms<APL, true>(ws, L, c, P.pp, e, lane);
     // world torsion axes (axis atoms' current positions)
+#pragma unroll 1
     for (int k = lane; k < c.nt; k += 32) {
         const int a0 = axs[k] & 0xffff, a1 = axs[k] >> 16;
         const float Ax = X[a0], Ay = X[AM + a0], Az = X[2 * AM + a0];
@@ -556,16 +531,23 @@ __device__ __forceinline__ float eval_eg(float* ws, const WSLayout& L, const flo
         tp[k] = make_float4(Ax - t0, Ay - t1, Az - t2, 0.f);
         tu[k] = make_float4(ux * nn, uy * nn, uz * nn, 0.f);
     }
-    // each atom's force with its torsion bitmask, and its torque (X - t) x F
+    // each atom's force with its torsion bitmask, and its torque (X - t) x F (in place of the forces)
     float4* FA = (float4*)(ws + L.FT);
     float4* TA = FA + AM;
+    float3 F[APL];
+#pragma unroll
+    for (int i = 0; i < APL; ++i) {
+        const int a = lane + 32 * i;
+        F[i] = make_float3(FF[a], FF[AM + a], FF[2 * AM + a]);
+    }
+    __syncwarp();
 #pragma unroll
     for (int i = 0; i < APL; ++i) {
         const int a = lane + 32 * i;
         if (a < c.na) {
             const float Fx = F[i].x, Fy = F[i].y, Fz = F[i].z;
             const float dx = X[a] - t0, dy = X[AM + a] - t1, dz = X[2 * AM + a] - t2;
-            FA[a] = make_float4(Fx, Fy, Fz, __uint_as_float(c.mask[i]));
+            FA[a] = make_float4(Fx, Fy, Fz, __uint_as_float(c.masks[a]));
             TA[a] = make_float4(dy * Fz - dz * Fy, dz * Fx - dx * Fz, dx * Fy - dy * Fx, 0.f);
         }
     }
@@ -604,6 +586,7 @@ __device__ __forceinline__ float eval_eg(float* ws, const WSLayout& L, const flo
             }
         }
     } else {
+#pragma unroll 1
         for (int k = lane; k <= c.nt; k += 32) {
             float S0 = 0.f, S1 = 0.f, S2 = 0.f, T0 = 0.f, T1 = 0.f, T2 = 0.f;
             const bool all = (k == c.nt);
@@ -630,6 +613,7 @@ __device__ __forceinline__ float eval_eg(float* ws, const WSLayout& L, const flo
 }
 
 __device__ __forceinline__ void wcopy(float* dst, const float* src, int D, int lane) {
+#pragma unroll 1
     for (int i = lane; i < D; i += 32) dst[i] = src[i];
     __syncwarp();
 }
@@ -640,6 +624,7 @@ __device__ __forceinline__ void conf_step(float* xn, const float* x, const float
         xn[3] = x[3]; xn[4] = x[4]; xn[5] = x[5]; xn[6] = x[6];
         quat_apply_rotvec(xn + 3, alpha * V[3].x, alpha * V[4].x, alpha * V[5].x);
     }
+#pragma unroll 1
     for (int k = lane; k < nt; k += 32) xn[7 + k] = x[7 + k] + alpha * V[6 + k].x;
     __syncwarp();
 }
@@ -649,6 +634,7 @@ template <int v>
 __device__ __forceinline__ float neg_hv(const float* H, const float4* V, int i, int D) {
     float a0 = 0.f, a1 = 0.f;
     int j = 0;
+#pragma unroll 2
     for (; j + 1 < D; j += 2) {
         a0 += H[j * D + i] * (v == 2 ? V[j].z : V[j].w);
         a1 += H[(j + 1) * D + i] * (v == 2 ? V[j + 1].z : V[j + 1].w);
@@ -681,6 +667,7 @@ __device__ __forceinline__ float bfgs(float* ws, const WSLayout& L, float* x, in
     int step = 0, trial = 0;
     bool first = true, again = false;
     while (true) {
+        if (!first && !again) conf_step(xn, x, V, alpha, c.nt, lane);
         const bool grad = first || again || trial == 0 || trial == 9;
         const float f = eval_eg<APL, GT, EX>(ws, L, first ? x : xn, first ? g : gn, c, P, tt, lane, grad);
         if (!again) ++n_eval;
@@ -689,10 +676,15 @@ __device__ __forceinline__ float bfgs(float* ws, const WSLayout& L, float* x, in
             f0 = f_orig = f;
             wcopy(xo, x, S, lane);
             float s = 0.f;
+#pragma unroll 1
             for (int i = lane; i < D; i += 32) {
                 go[i] = g[i];
                 float a0 = 0.f, a1 = 0.f;   // p = -H g with H the identity
-                for (int j = 0; j < D; ++j) (j & 1 ? a1 : a0) += (i == j ? 1.f : 0.f) * g[j];
+#pragma unroll 1
+                for (int j = 0; j < D; j += 2) {
+                    a0 += (i == j ? 1.f : 0.f) * g[j];
+                    if (j + 1 < D) a1 += (i == j + 1 ? 1.f : 0.f) * g[j + 1];
+                }
                 const float pi = -(a0 + a1);
                 V[i].x = pi;
                 s += pi * g[i];
@@ -700,7 +692,6 @@ __device__ __forceinline__ float bfgs(float* ws, const WSLayout& L, float* x, in
             __syncwarp();
             if (iters <= 0) break;
             pg = warp_sum(s);
-            conf_step(xn, x, V, alpha, c.nt, lane);
             continue;
         }
         // Armijo test (c = 1e-4); up to 10 trials halving alpha. After a 10th failed trial the last point is taken
@@ -709,11 +700,9 @@ __device__ __forceinline__ float bfgs(float* ws, const WSLayout& L, float* x, in
         if (!again) {
             if (!(f - f0 < 1e-4f * alpha * pg)) {
                 alpha *= 0.5f;
-                if (++trial < 10) {
-                    conf_step(xn, x, V, alpha, c.nt, lane);
-                    continue;
-                }
+                if (++trial < 10) continue;
                 stuck = true;
+#pragma unroll 1
                 for (int i = lane; i < S; i += 32) stuck = stuck && __float_as_int(x[i]) == __float_as_int(xn[i]);
                 stuck = __all_sync(0xffffffffu, stuck);
             } else if (!grad) {
@@ -726,9 +715,11 @@ __device__ __forceinline__ float bfgs(float* ws, const WSLayout& L, float* x, in
         // would repeat this one.
         if (stuck) break;
         f0 = f;
+#pragma unroll 1
         for (int i = lane; i < S; i += 32) x[i] = xn[i];
         float gg = 0.f, yy = 0.f;
         double yp = 0.0;
+#pragma unroll 1
         for (int i = lane; i < D; i += 32) {
             const float gi = gn[i], yi = gi - g[i];
             gg += gi * gi;
@@ -745,13 +736,16 @@ __device__ __forceinline__ float bfgs(float* ws, const WSLayout& L, float* x, in
         if (!(sqrtf(gg) >= 1e-5f)) break;
         if (step == 0) {   // H: the identity, rescaled from the first step's curvature
             const float dg = fabsf(yy) > EPSF ? (float)((double)alpha * yp / (double)yy) : 1.f;
+#pragma unroll 1
             for (int i = lane; i < D; i += 32)
+#pragma unroll 2
                 for (int j = 0; j < D; ++j) H[j * D + i] = (i == j) ? dg : 0.f;
             __syncwarp();
         }
         const double ayp = (double)alpha * yp;
         float s = 0.f;
         if (ayp >= (double)EPSF) {
+#pragma unroll 1
             for (int i = lane; i < D; i += 32) {
                 const float mi = neg_hv<2>(H, V, i, D);
                 V[i].y = mi;
@@ -772,6 +766,7 @@ __device__ __forceinline__ float bfgs(float* ws, const WSLayout& L, float* x, in
                 if (i < D) {
                     const float mi = V[i].y, pi = V[i].x;
                     float a0 = 0.f, a1 = 0.f;
+#pragma unroll 2
                     for (int j = 0; j < D; ++j) {
                         const float4 v = V[j];
                         float hij = H[j * D + i];
@@ -787,6 +782,7 @@ __device__ __forceinline__ float bfgs(float* ws, const WSLayout& L, float* x, in
             if (lane < D) V[lane].x = pn[0];
             if (lane + 32 < D) V[lane + 32].x = pn[1];
         } else {
+#pragma unroll 1
             for (int i = lane; i < D; i += 32) {
                 const float pi = neg_hv<3>(H, V, i, D);
                 s += pi * V[i].w;
@@ -798,7 +794,6 @@ __device__ __forceinline__ float bfgs(float* ws, const WSLayout& L, float* x, in
         pg = warp_sum(s);
         alpha = 1.f;
         trial = 0;
-        conf_step(xn, x, V, alpha, c.nt, lane);
     }
     if (!(f0 <= f_orig)) {
         f0 = f_orig;
@@ -958,7 +953,7 @@ __global__ void __launch_bounds__(128, MINB) mc_kernel(const __grid_constant__ S
         Chain<APL> c;
         const int* nb = M.nbr ? M.nbr + (long long)ch * M.nb_max : nullptr;
         const int nbn = M.nbr ? M.nbr_n[ch] : 0;
-        load_chain<APL, GT>(c, P, tt, l, ws, L, lane, M.exact, nb, nbn);
+        load_chain<APL, GT>(c, P, tt, l, ws, L, lane, nb, nbn);
         const int S = 7 + c.nt;
         const int iters = M.bfgs_iters > 0 ? M.bfgs_iters : (25 + c.na) / 3;
         float* cur = ws + L.cur;
@@ -1095,7 +1090,7 @@ __global__ void __launch_bounds__(128) eg_kernel(const __grid_constant__ SearchP
     for (int ch = blockIdx.x * (blockDim.x >> 5) + wid; ch < n; ch += warps) {
         const int l = chain_lig[ch];
         Chain<APL> c;
-        load_chain<APL, GT>(c, P, tt, l, ws, L, lane, exact, nullptr, 0);
+        load_chain<APL, GT>(c, P, tt, l, ws, L, lane, nullptr, 0);
         float* x = ws + L.x;
         float* g = ws + L.g;
         for (int i = lane; i < SDM; i += 32) x[i] = state[(long long)ch * SDM + i];

@@ -91,8 +91,9 @@ typedef struct {
     void* atoms;               /* [L, AM] float4: ref xyz + (gslot | typ << 16) bits */
     void* masks;               /* [L, AM] uint32 torsion bitmask of each atom (KM <= 32) */
     void* tors;                /* [L, KM, 2] float4: axp + ax0 bits, axu + ax1 bits */
-    void* pairs;               /* [L, ceil(P/32)*32] int2: (i | j << 8 | flags << 16, radius-sum bits), scheduled
-                                  in rounds of 32 with no atom twice per round where possible; empty slots -1 */
+    void* pairs;               /* [L, ceil(P/32)*32] int2: (i | j << 8 | flags << 16 | links of the round's slots with
+                                  the same atoms, the round's repeat counts), scheduled in rounds of 32 with no atom
+                                  twice per round where possible; empty slots: x = -1 */
     void* info;                /* [L] int4: na, nt, np, rec_idx */
     void* rg;                  /* [L] float */
 } adock_work_t;
