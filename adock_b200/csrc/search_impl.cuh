@@ -1096,7 +1096,7 @@ __global__ void __launch_bounds__(128) eg_kernel(const __grid_constant__ SearchP
         for (int i = lane; i < SDM; i += 32) x[i] = state[(long long)ch * SDM + i];
         __syncwarp();
         const float e = eval_eg<APL, GT, EX>(ws, L, x, g, c, P, tt, lane, true);
-        for (int i = lane; i < 6 + c.nt; i += 32) g_out[(long long)ch * DMM + i] = g[i];
+        for (int i = lane; i < DMM; i += 32) g_out[(long long)ch * DMM + i] = i < 6 + c.nt ? g[i] : 0.f;
         if (lane == 0) e_out[ch] = e;
         __syncwarp();
     }

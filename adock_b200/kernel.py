@@ -114,8 +114,8 @@ class B200KernelProblem:
     def energy_grad(self, chain_lig, state, exact=False):
         """chain_lig int32 [N], state [N, SD] -> (e [N], g [N, DM])."""
         N = state.shape[0]
-        e = torch.zeros(N, device=self.device)
-        g = torch.zeros(N, self.DM, device=self.device)
+        e = torch.empty(N, device=self.device)
+        g = torch.empty(N, self.DM, device=self.device)   # the kernel writes whole rows
         if exact:
             assert self.c_rec.RN > 0, "exact mode needs receptor atoms (Problem.rec)"
         cl = self._i32(chain_lig)

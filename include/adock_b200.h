@@ -189,7 +189,7 @@ int adock_grid_convert(const float* src, void* dst, long long n, int dtype, void
 int adock_prepare(const adock_ligands_t* lig, const adock_sf_t* sf, adock_work_t* work, void* stream);
 
 /* Energy + analytic pose gradient of N states: replaces eg_kernel (mckernel.py:411-447) /
- * KernelProblem.energy_grad (mckernel.py:652-660). state [N, 7+KM], e [N], g [N, 6+KM] (dev). */
+ * KernelProblem.energy_grad (mckernel.py:652-660). state [N, 7+KM], e [N], g [N, 6+KM] (dev; 0 past a ligand's torsions). */
 int adock_eg(const adock_ligands_t* lig, const adock_work_t* work, const adock_grids_t* grids,
              const adock_sf_t* sf, const adock_receptors_t* rec, const int* chain_lig, int n, const float* state,
              float* e_out, float* g_out, int exact, void* stream);
