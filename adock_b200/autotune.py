@@ -5,9 +5,10 @@ resident 128-thread blocks per SM, i.e. 128, 80 or 64 registers). Which is faste
 (AM), the torsion bucket (KM), the map storage type and the GPU. ``tune_mc`` brings the batch's chains (up to 16,384)
 into the regime of a running search (optimised starts + 8 MC steps), then times 8 and 32 MC steps under each
 variant and keeps the one with the least time per step between the two; results are cached per (device name, AM,
-KM, map dtype) for the life of the process and in ``$ADOCK_TUNE_CACHE`` (a JSON file) if set. A launch of the
-80-register variant has about 5 ms more fixed cost than the 128-register one and less per step (2.79 vs 2.93 ms on
-the 256-ligand batch), so the time of one short sample picked the variant that a 2,000-step search ran 8 % slower.
+KM, map dtype) for the life of the process and in ``$ADOCK_TUNE_CACHE`` (a JSON file) if set. The
+variants' order follows the kernel's code: on the 256-ligand batch the 128-register variant now takes 1.44 ms per step,
+the others 2.22 and 2.44 ms. The two run lengths take out a launch's fixed part (ramp-up and tail), which differs between
+variants and would decide the time of one short sample.
 """
 from __future__ import annotations
 
