@@ -38,9 +38,9 @@ enum { NEED_HYD = 1, NEED_HB = 2 };
 
 struct VinaPrm {
     float cutoff, rep_off;
-    float g1_k, g1_c, g2_k, g2_c;        // Gaussian = 2^-(k d - c)^2
-    float hyd_k, hyd_c, hb_k, hb_c;      // ramp = saturate(c - k d)
-    int falling;                         // a ramp has k < 0: not 0 far away
+    float g1_off, g1_k, g2_off, g2_k;         // Gaussian = 2^-((d - off) k)^2
+    float hyd_bad, hyd_inv, hb_bad, hb_inv;   // ramp = saturate((bad - d) inv); a step (good = bad) has inv = infinity
+    int falling;                              // a ramp has inv < 0: not 0 far away
     float w[5];
     int n_lt, n_xs, n_rad;
     float rad[24];       // distinct radii, ascending
@@ -53,7 +53,7 @@ struct VinaPrm {
 
 struct FitPrm {
     float cutoff, rep_off;
-    float g1_k, g1_c, g2_k, g2_c, hyd_k, hyd_c, hb_k, hb_c;   // as VinaPrm
+    float g1_off, g1_k, g2_off, g2_k, hyd_bad, hyd_inv, hb_bad, hb_inv;   // as VinaPrm
     int falling;
     float ion_rmin, ion_cut, rep_cap;                          // ion_rmin = 1 / minimum distance, ion_cut = 1 / cutoff^2
     int n_lt, n_rt;
@@ -223,7 +223,7 @@ struct Distances {
 
 // Vina maps. Bound by instruction issue and the two exponentials per (atom, point, radius). A thread per point that
 // added five sums per ligand type and tested every staged atom took 687 us for 8,000 receptor atoms, 81^3 points and 8
-// types (4 radii), this 295 us.
+// types (4 radii), this 303 us.
 // PER_TERM writes the five unweighted terms: the first two sums then hold one of the first three per sweep.
 template <int PP, bool PER_TERM>
 __global__ void __launch_bounds__(Tile<PP>::THREADS, PP == 2 ? 3 : 8) grid_vina_kernel(const float* __restrict__ rxyz,
@@ -287,19 +287,19 @@ __global__ void __launch_bounds__(Tile<PP>::THREADS, PP == 2 ? 3 : 8) grid_vina_
 #pragma unroll
                             for (int h = 0; h < PP; ++h) {
                                 const float d = r[h] - P.rad[r0 + q];
-                                const float u1 = d * P.g1_k - P.g1_c, u2 = d * P.g2_k - P.g2_c;
+                                const float u1 = (d - P.g1_off) * P.g1_k, u2 = (d - P.g2_off) * P.g2_k;
                                 const float dr = fminf(d - P.rep_off, 0.f);
                                 float* a = sum[h][q];
                                 a[SUM_REP] += w3 * dr * dr;
                                 a[SUM_GAUSS] += w1 * exp2_ftz(-u1 * u1);
                                 a[SUM_GAUSS] += w2 * exp2_ftz(-u2 * u2);
                                 if (need & NEED_HYD) {
-                                    float hyd = __saturatef(P.hyd_c - d * P.hyd_k);
+                                    float hyd = __saturatef((P.hyd_bad - d) * P.hyd_inv);
                                     if (P.falling) hyd *= on[h];
                                     a[SUM_HYD] += hyd * g.x;
                                 }
                                 if (need & NEED_HB) {
-                                    float hb = __saturatef(P.hb_c - d * P.hb_k);
+                                    float hb = __saturatef((P.hb_bad - d) * P.hb_inv);
                                     if (P.falling) hb *= on[h];
                                     a[SUM_DON] += hb * g.y;
                                     a[SUM_ACC] += hb * g.z;
@@ -341,7 +341,7 @@ __global__ void __launch_bounds__(Tile<PP>::THREADS, PP == 2 ? 3 : 8) grid_vina_
 
 // Fitted maps. Bound by instruction issue: six multiply-adds per (atom, point, type) beside the basis per radius; the
 // weights come from shared memory, once for a thread's two points. One point per thread with every staged atom tested took
-// 732 us for 8,000 receptor atoms, 81^3 points and 8 types, this 421 us.
+// 732 us for 8,000 receptor atoms, 81^3 points and 8 types, this 436 us.
 // Packed FP32 pairs for the two points (fma.rn.f32x2) were slower in both kernels (287 and 432 us): the exponentials, minima
 // and ramps stay scalar, so the registers and moves of the pairs cost more than the issue slots they save.
 template <int PP>
@@ -415,13 +415,13 @@ __global__ void __launch_bounds__(Tile<PP>::THREADS, PP == 2 ? 3 : 6) grid_fit_k
 #pragma unroll
                             for (int h = 0; h < PP; ++h) {
                                 const float d = r[h] - P.rad_lig[q0 + q];
-                                const float u1 = d * P.g1_k - P.g1_c, u2 = d * P.g2_k - P.g2_c;
+                                const float u1 = (d - P.g1_off) * P.g1_k, u2 = (d - P.g2_off) * P.g2_k;
                                 const float dr = fminf(d - P.rep_off, 0.f);
                                 g1[h] = exp2_ftz(-u1 * u1);
                                 g2[h] = exp2_ftz(-u2 * u2);
                                 rep[h] = fminf(dr * dr, P.rep_cap);
-                                hyd[h] = __saturatef(P.hyd_c - d * P.hyd_k);
-                                hb[h] = __saturatef(P.hb_c - d * P.hb_k);
+                                hyd[h] = __saturatef((P.hyd_bad - d) * P.hyd_inv);
+                                hb[h] = __saturatef((P.hb_bad - d) * P.hb_inv);
                                 if (P.falling) { hyd[h] *= on[h]; hb[h] *= on[h]; }
                             }
                         }
@@ -505,17 +505,11 @@ static bool two_points(const Cells& C, float cutoff, float spacing, int nx, int 
     return (long long)g.x * g.y * g.z >= 2LL * sm_count() && (!C.start || tile_reach(C, 8, cutoff, spacing) <= MAX_COLUMNS);
 }
 
-// Gaussian exp(-((d - off) / w)^2) = 2^-(k d - c)^2 and ramp (bad - d) / (bad - good) = c - k d
-static void gauss_prm(float off, float w, float& k, float& c) {
-    const double s = sqrt(1.4426950408889634) / (double)w;
-    k = (float)s;
-    c = (float)(s * (double)off);
-}
-static void ramp_prm(float good, float bad, float& k, float& c) {
-    const double s = 1.0 / ((double)bad - (double)good);
-    k = (float)s;
-    c = (float)(s * (double)bad);
-}
+// exp(-((d - off) / w)^2) = 2^-((d - off) k)^2 and the ramp's slope 1 / (bad - good). The offsets stay apart from the
+// products: folded into one multiply-add (k d - c) a step's or a zero width's infinite k would meet an infinite c and give
+// NaN. The extra instruction per term costs 3 % (8,000 atoms, 81^3 points, 8 types: 295 us folded, 303 us so).
+static float gauss_k(float w) { return (float)(sqrt(1.4426950408889634) / (double)w); }
+static float ramp_inv(float good, float bad) { return (float)(1.0 / ((double)bad - (double)good)); }
 
 static int grid_vina_launch(const float* rec_xyz, const int* rec_types, int n_rec, const Cells& C, const float* radius,
                             const int* hyd, const int* don, const int* acc, int n_xs, const int* lig_types, int n_lt,
@@ -531,12 +525,12 @@ static int grid_vina_launch(const float* rec_xyz, const int* rec_types, int n_re
     if (rc) return rc;
     VinaPrm P;
     P.cutoff = prm[0];
-    gauss_prm(prm[1], prm[2], P.g1_k, P.g1_c);
-    gauss_prm(prm[3], prm[4], P.g2_k, P.g2_c);
+    P.g1_off = prm[1]; P.g1_k = gauss_k(prm[2]);
+    P.g2_off = prm[3]; P.g2_k = gauss_k(prm[4]);
     P.rep_off = prm[5];
-    ramp_prm(prm[6], prm[7], P.hyd_k, P.hyd_c);
-    ramp_prm(prm[8], prm[9], P.hb_k, P.hb_c);
-    P.falling = !(P.hyd_k > 0.f && P.hb_k > 0.f);
+    P.hyd_bad = prm[7]; P.hyd_inv = ramp_inv(prm[6], prm[7]);
+    P.hb_bad = prm[9]; P.hb_inv = ramp_inv(prm[8], prm[9]);
+    P.falling = !(P.hyd_inv > 0.f && P.hb_inv > 0.f);
     for (int m = 0; m < 5; ++m) P.w[m] = prm[10 + m];
     P.n_lt = n_lt; P.n_xs = n_xs;
     for (int q = 0; q < n_lt; ++q) ADOCK_CHECK_ARG(lig_types[q] >= 0 && lig_types[q] < n_xs, "ligand type out of range");
@@ -605,12 +599,12 @@ static int grid_fit_launch(const float* rec_xyz, const int* rec_ext, int n_rec, 
     if (rc) return rc;
     FitPrm P;
     P.cutoff = prm[0];
-    gauss_prm(prm[1], prm[2], P.g1_k, P.g1_c);
-    gauss_prm(prm[3], prm[4], P.g2_k, P.g2_c);
+    P.g1_off = prm[1]; P.g1_k = gauss_k(prm[2]);
+    P.g2_off = prm[3]; P.g2_k = gauss_k(prm[4]);
     P.rep_off = prm[5];
-    ramp_prm(prm[6], prm[7], P.hyd_k, P.hyd_c);
-    ramp_prm(prm[8], prm[9], P.hb_k, P.hb_c);
-    P.falling = !(P.hyd_k > 0.f && P.hb_k > 0.f);
+    P.hyd_bad = prm[7]; P.hyd_inv = ramp_inv(prm[6], prm[7]);
+    P.hb_bad = prm[9]; P.hb_inv = ramp_inv(prm[8], prm[9]);
+    P.falling = !(P.hyd_inv > 0.f && P.hb_inv > 0.f);
     P.ion_rmin = prm[10] > 0.f ? 1.f / prm[10] : INFINITY; P.ion_cut = 1.f / (prm[0] * prm[0]); P.rep_cap = prm[11];
     P.n_lt = n_lt; P.n_rt = n_rt;
     int order[64];
