@@ -11,7 +11,7 @@
 // CTA, and the summation order per point is the reference's receptor order; with one, it is the cell order.
 //
 // The distance-dependent parts of the terms depend on the ligand type only through its radius. The Vina kernel keeps
-// sums per distinct radius (the weighted Gaussians and repulsion; the hydrophobic ramp over hydrophobic atoms; the
+// sums per distinct radius (the Gaussians and the repulsion; the hydrophobic ramp over hydrophobic atoms; the
 // hydrogen-bond ramp over donors, acceptors and either) and forms every type's map from them at the end; the fitted
 // kernel evaluates the basis once per distinct radius and adds it with each type's weights. Radii (types) are processed
 // in groups that fit the registers.
@@ -31,9 +31,10 @@ struct Tile {
     static constexpr int WARPS = X * Y * Z / (32 * PP), THREADS = 32 * WARPS;
 };
 
-// Sums of one distinct radius that a map needs. The repulsion has a sum of its own: few atoms overlap a point, and adding
-// everybody's small Gaussians to a large repulsion would round each time.
-enum { SUM_REP, SUM_GAUSS, SUM_HYD, SUM_DON, SUM_ACC, SUM_EITHER, SUMS };
+// Sums of one distinct radius that a map needs, without the weights: each term's rounding then stays in proportion to the
+// term (everybody's small Gaussians added to a large repulsion would round each time), and the same sums give the
+// per-term maps.
+enum { SUM_G1, SUM_G2, SUM_REP, SUM_HYD, SUM_DON, SUM_ACC, SUM_EITHER, SUMS };
 enum { NEED_HYD = 1, NEED_HB = 2 };
 
 struct VinaPrm {
@@ -43,10 +44,11 @@ struct VinaPrm {
     int falling;                              // a ramp has inv < 0: not 0 far away
     float w[5];
     int n_lt, n_xs, n_rad;
+    int per_term;        // write the five unweighted terms
     float rad[24];       // distinct radii, ascending
     int need[24];        // NEED_* of the radius's types
     int rad_of[24];      // each map's radius
-    int gate[24];        // each map's sums beside the first two: bit 0 SUM_HYD; bits 1-2 the H-bond sum (0 none)
+    int gate[24];        // each map's sums beside the first three: bit 0 SUM_HYD; bits 1-2 the H-bond sum (0 none)
     float radius[64];
     int flags[64];  // bit0 hydrophobic, bit1 donor, bit2 acceptor
 };
@@ -223,9 +225,8 @@ struct Distances {
 
 // Vina maps. Bound by instruction issue and the two exponentials per (atom, point, radius). A thread per point that
 // added five sums per ligand type and tested every staged atom took 687 us for 8,000 receptor atoms, 81^3 points and 8
-// types (4 radii), this 303 us.
-// PER_TERM writes the five unweighted terms: the first two sums then hold one of the first three per sweep.
-template <int PP, bool PER_TERM>
+// types (4 radii), this 294 us, the per-term maps 304 us.
+template <int PP>
 __global__ void __launch_bounds__(Tile<PP>::THREADS, PP == 2 ? 3 : 8) grid_vina_kernel(const float* __restrict__ rxyz,
                                                                       const int* __restrict__ rtype, int n_rec,
                                                                       const __grid_constant__ Cells C, float ox, float oy,
@@ -240,98 +241,96 @@ __global__ void __launch_bounds__(Tile<PP>::THREADS, PP == 2 ? 3 : 8) grid_vina_
     const int lane = threadIdx.x & 31, total = col_off[ncol];
     const float cut2 = P.cutoff * P.cutoff, reach2 = cut2 * 1.0001f + 1e-3f;
     const long long npts = (long long)nx * ny * nz;
-    for (int term = 0; term < (PER_TERM ? 3 : 1); ++term) {
-        const float w1 = PER_TERM ? (term == 0 ? 1.f : 0.f) : P.w[0], w2 = PER_TERM ? (term == 1 ? 1.f : 0.f) : P.w[1],
-                    w3 = PER_TERM ? (term == 2 ? 1.f : 0.f) : P.w[2];
-        for (int r0 = 0; r0 < P.n_rad; r0 += RADIUS_GROUP) {
-            float sum[PP][RADIUS_GROUP][SUMS];
+    for (int r0 = 0; r0 < P.n_rad; r0 += RADIUS_GROUP) {
+        float sum[PP][RADIUS_GROUP][SUMS];
 #pragma unroll
-            for (int h = 0; h < PP; ++h)
+        for (int h = 0; h < PP; ++h)
 #pragma unroll
-                for (int q = 0; q < RADIUS_GROUP; ++q)
+            for (int q = 0; q < RADIUS_GROUP; ++q)
 #pragma unroll
-                    for (int m = 0; m < SUMS; ++m) sum[h][q][m] = 0.f;
-            int start = 0;
-            while (start < total) {
-                int cnt;
-                start = stage_atoms<Tile<PP>::THREADS>(rxyz, rtype, col_begin, col_off, ncol, start, t.lo, t.hi, &cnt, wsum,
-                                                       [&](int s, float ax, float ay, float az, int ta) {
-                                                           const int f = P.flags[ta];
-                                                           S[s] = make_float4(ax, ay, az, P.radius[ta]);
-                                                           G[s] = make_float4(f & 1 ? 1.f : 0.f, f & 2 ? 1.f : 0.f,
-                                                                              f & 4 ? 1.f : 0.f, f & 6 ? 1.f : 0.f);
-                                                       });
-                for (int s0 = 0; s0 < cnt; s0 += 32) {
-                    const int s = s0 + lane;
-                    bool near = false;
-                    if (s < cnt) {
-                        const float4 A = S[s];
-                        near = t.in_reach(A.x, A.y, A.z, reach2);
+                for (int m = 0; m < SUMS; ++m) sum[h][q][m] = 0.f;
+        int start = 0;
+        while (start < total) {
+            int cnt;
+            start = stage_atoms<Tile<PP>::THREADS>(rxyz, rtype, col_begin, col_off, ncol, start, t.lo, t.hi, &cnt, wsum,
+                                                   [&](int s, float ax, float ay, float az, int ta) {
+                                                       const int f = P.flags[ta];
+                                                       S[s] = make_float4(ax, ay, az, P.radius[ta]);
+                                                       G[s] = make_float4(f & 1 ? 1.f : 0.f, f & 2 ? 1.f : 0.f,
+                                                                          f & 4 ? 1.f : 0.f, f & 6 ? 1.f : 0.f);
+                                                   });
+            for (int s0 = 0; s0 < cnt; s0 += 32) {
+                const int s = s0 + lane;
+                bool near = false;
+                if (s < cnt) {
+                    const float4 A = S[s];
+                    near = t.in_reach(A.x, A.y, A.z, reach2);
+                }
+                unsigned todo = __ballot_sync(0xffffffffu, near);
+                while (todo) {
+                    const int at = s0 + __ffs(todo) - 1;
+                    todo &= todo - 1;
+                    const float4 A = S[at], g = G[at];
+                    const Distances<PP> D(A.x, t.x, A.y - t.y, A.z - t.z, cut2);
+                    float r[PP], on[PP];
+#pragma unroll
+                    for (int h = 0; h < PP; ++h) {
+                        r[h] = D.far[h] ? FAR_AWAY : D.r[h] - A.w;
+                        on[h] = D.far[h] ? 0.f : 1.f;
                     }
-                    unsigned todo = __ballot_sync(0xffffffffu, near);
-                    while (todo) {
-                        const int at = s0 + __ffs(todo) - 1;
-                        todo &= todo - 1;
-                        const float4 A = S[at], g = G[at];
-                        const Distances<PP> D(A.x, t.x, A.y - t.y, A.z - t.z, cut2);
-                        float r[PP], on[PP];
+#pragma unroll
+                    for (int q = 0; q < RADIUS_GROUP; ++q) {
+                        if (r0 + q >= P.n_rad) break;
+                        const int need = P.need[r0 + q];
 #pragma unroll
                         for (int h = 0; h < PP; ++h) {
-                            r[h] = D.far[h] ? FAR_AWAY : D.r[h] - A.w;
-                            on[h] = D.far[h] ? 0.f : 1.f;
-                        }
-#pragma unroll
-                        for (int q = 0; q < RADIUS_GROUP; ++q) {
-                            if (r0 + q >= P.n_rad) break;
-                            const int need = P.need[r0 + q];
-#pragma unroll
-                            for (int h = 0; h < PP; ++h) {
-                                const float d = r[h] - P.rad[r0 + q];
-                                const float u1 = (d - P.g1_off) * P.g1_k, u2 = (d - P.g2_off) * P.g2_k;
-                                const float dr = fminf(d - P.rep_off, 0.f);
-                                float* a = sum[h][q];
-                                a[SUM_REP] += w3 * dr * dr;
-                                a[SUM_GAUSS] += w1 * exp2_ftz(-u1 * u1);
-                                a[SUM_GAUSS] += w2 * exp2_ftz(-u2 * u2);
-                                if (need & NEED_HYD) {
-                                    float hyd = __saturatef((P.hyd_bad - d) * P.hyd_inv);
-                                    if (P.falling) hyd *= on[h];
-                                    a[SUM_HYD] += hyd * g.x;
-                                }
-                                if (need & NEED_HB) {
-                                    float hb = __saturatef((P.hb_bad - d) * P.hb_inv);
-                                    if (P.falling) hb *= on[h];
-                                    a[SUM_DON] += hb * g.y;
-                                    a[SUM_ACC] += hb * g.z;
-                                    a[SUM_EITHER] += hb * g.w;
-                                }
+                            const float d = r[h] - P.rad[r0 + q];
+                            const float u1 = (d - P.g1_off) * P.g1_k, u2 = (d - P.g2_off) * P.g2_k;
+                            const float dr = fminf(d - P.rep_off, 0.f);
+                            float* a = sum[h][q];
+                            a[SUM_G1] += exp2_ftz(-u1 * u1);
+                            a[SUM_G2] += exp2_ftz(-u2 * u2);
+                            a[SUM_REP] += dr * dr;
+                            if (need & NEED_HYD) {
+                                float hyd = __saturatef((P.hyd_bad - d) * P.hyd_inv);
+                                if (P.falling) hyd *= on[h];
+                                a[SUM_HYD] += hyd * g.x;
+                            }
+                            if (need & NEED_HB) {
+                                float hb = __saturatef((P.hb_bad - d) * P.hb_inv);
+                                if (P.falling) hb *= on[h];
+                                a[SUM_DON] += hb * g.y;
+                                a[SUM_ACC] += hb * g.z;
+                                a[SUM_EITHER] += hb * g.w;
                             }
                         }
                     }
                 }
-                __syncthreads();
             }
-            // the maps of these radii
-            for (int o = 0; o < P.n_lt; ++o) {
+            __syncthreads();
+        }
+        // the maps of these radii
+        for (int o = 0; o < P.n_lt; ++o) {
 #pragma unroll
-                for (int q = 0; q < RADIUS_GROUP; ++q) {
-                    if (P.rad_of[o] != r0 + q) continue;
-                    const int hb = P.gate[o] >> 1;
+            for (int q = 0; q < RADIUS_GROUP; ++q) {
+                if (P.rad_of[o] != r0 + q) continue;
+                const int hb = P.gate[o] >> 1;
 #pragma unroll
-                    for (int h = 0; h < PP; ++h) {
-                        if (t.p[h] < 0) continue;
-                        const float* a = sum[h][q];
-                        const float e_hyd = P.gate[o] & 1 ? a[SUM_HYD] : 0.f;
-                        const float e_hb = hb == 0 ? 0.f : (hb == 1 ? a[SUM_DON] : (hb == 2 ? a[SUM_ACC] : a[SUM_EITHER]));
-                        if (PER_TERM) {
-                            out[((long long)term * P.n_lt + o) * npts + t.p[h]] = a[SUM_REP] + a[SUM_GAUSS];
-                            if (term == 0) {
-                                out[((long long)3 * P.n_lt + o) * npts + t.p[h]] = e_hyd;
-                                out[((long long)4 * P.n_lt + o) * npts + t.p[h]] = e_hb;
-                            }
-                        } else {
-                            out[(long long)o * npts + t.p[h]] = a[SUM_REP] + a[SUM_GAUSS] + P.w[3] * e_hyd + P.w[4] * e_hb;
-                        }
+                for (int h = 0; h < PP; ++h) {
+                    if (t.p[h] < 0) continue;
+                    const float* a = sum[h][q];
+                    const float e_hyd = P.gate[o] & 1 ? a[SUM_HYD] : 0.f;
+                    const float e_hb = hb == 0 ? 0.f : (hb == 1 ? a[SUM_DON] : (hb == 2 ? a[SUM_ACC] : a[SUM_EITHER]));
+                    const float e[5] = {a[SUM_G1], a[SUM_G2], a[SUM_REP], e_hyd, e_hb};
+                    float* dst = out + (long long)o * npts + t.p[h];
+                    if (P.per_term) {
+#pragma unroll
+                        for (int m = 0; m < 5; ++m) dst[(long long)m * P.n_lt * npts] = e[m];
+                    } else {
+                        float v = 0.f;
+#pragma unroll
+                        for (int m = 0; m < 5; ++m) v += P.w[m] * e[m];
+                        *dst = v;
                     }
                 }
             }
@@ -532,7 +531,7 @@ static int grid_vina_launch(const float* rec_xyz, const int* rec_types, int n_re
     P.hb_bad = prm[9]; P.hb_inv = ramp_inv(prm[8], prm[9]);
     P.falling = !(P.hyd_inv > 0.f && P.hb_inv > 0.f);
     for (int m = 0; m < 5; ++m) P.w[m] = prm[10 + m];
-    P.n_lt = n_lt; P.n_xs = n_xs;
+    P.n_lt = n_lt; P.n_xs = n_xs; P.per_term = per_term;
     for (int q = 0; q < n_lt; ++q) ADOCK_CHECK_ARG(lig_types[q] >= 0 && lig_types[q] < n_xs, "ligand type out of range");
     float rl[24];
     int order[24];
@@ -561,14 +560,11 @@ static int grid_vina_launch(const float* rec_xyz, const int* rec_types, int n_re
     const dim3 small = tiles<1>(nx, ny, nz);
     ADOCK_CHECK_ARG(small.y < 65536 && small.z < 65536, "grid too large");
     cudaStream_t st = (cudaStream_t)stream;
-    if (per_term)
-        grid_vina_kernel<1, true><<<small, Tile<1>::THREADS, 0, st>>>(rec_xyz, rec_types, n_rec, C, ox, oy, oz, spacing, nx,
-                                                                      ny, nz, P, out);
-    else if (two_points(C, prm[0], spacing, nx, ny, nz))
-        grid_vina_kernel<2, false><<<tiles<2>(nx, ny, nz), Tile<2>::THREADS, 0, st>>>(rec_xyz, rec_types, n_rec, C, ox, oy, oz,
+    if (two_points(C, prm[0], spacing, nx, ny, nz))
+        grid_vina_kernel<2><<<tiles<2>(nx, ny, nz), Tile<2>::THREADS, 0, st>>>(rec_xyz, rec_types, n_rec, C, ox, oy, oz,
                                                                                       spacing, nx, ny, nz, P, out);
     else
-        grid_vina_kernel<1, false><<<small, Tile<1>::THREADS, 0, st>>>(rec_xyz, rec_types, n_rec, C, ox, oy, oz, spacing, nx,
+        grid_vina_kernel<1><<<small, Tile<1>::THREADS, 0, st>>>(rec_xyz, rec_types, n_rec, C, ox, oy, oz, spacing, nx,
                                                                        ny, nz, P, out);
     ADOCK_CUDA(cudaGetLastError());
     return ADOCK_OK;
