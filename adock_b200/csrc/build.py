@@ -22,7 +22,7 @@ LINK = ["-shared", "-cudart", "shared"]
 
 def _digest():
     h = hashlib.sha1()
-    for f in SOURCES + ["common.cuh", "search_impl.cuh"]:
+    for f in SOURCES + ["common.cuh", "search_impl.cuh", "mma_ring.h"]:
         h.update((HERE / f).read_bytes())
     h.update((ROOT / "include" / "adock_b200.h").read_bytes())
     h.update(" ".join(FLAGS).encode())

@@ -15,6 +15,7 @@
 // adock_mlp_forward and adock_mlp_loss_grad queue a whole forward pass, or forward and backward pass, from one call:
 // the layers are a few microseconds each, so the launches' host cost would otherwise decide.
 #include "common.cuh"
+#include "mma_ring.h"
 
 namespace adock {
 
@@ -361,50 +362,47 @@ __global__ void __launch_bounds__(TC_THREADS, 2) gemm_bf16_tc_kernel(const __gri
         b.load(g.B, g.sBn, g.sBk, n0, g.N, kt * TC_BK, g.K, b_mode, TC_THREADS / 2);
     };
     if (steps > 0) load(k_begin);
-    bool ok = true;
-    for (int it = 0; it < steps && ok; ++it) {
-        const int k0 = (k_begin + it) * TC_BK, s = it % TC_STAGES;
+    auto wait = [&](int s, unsigned parity) { return tc_wait(smem_u32(&mbar[s]), parity); };
+    auto fill = [&](int it, int s) {
+        const int k0 = (k_begin + it) * TC_BK;
         unsigned char* As = tc_smem + s * SM::STAGE;
-        unsigned char* Bs = As + SM::A;
-        if (it >= TC_STAGES && !tc_wait(smem_u32(&mbar[s]), (uint32_t)((it / TC_STAGES - 1) & 1))) atomicExch(&fail_sh, 1);
         a.store(As, g.A, g.sAm, g.sAk, m0, g.M, k0, g.K, a_mode, 0);
-        b.store(Bs, g.B, g.sBn, g.sBk, n0, g.N, k0, g.K, b_mode, TC_THREADS / 2);
+        b.store(As + SM::A, g.B, g.sBn, g.sBk, n0, g.N, k0, g.K, b_mode, TC_THREADS / 2);
         if (it + 1 < steps) load(k_begin + it + 1);
-        // make the generic-proxy stores visible to the tensor core (async proxy), then one thread issues the MMAs
+        // make the generic-proxy stores visible to the tensor core (async proxy) before the barrier
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        __syncthreads();
-        ok = fail_sh == 0;
-        if (tid == 0 && ok) {
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            const uint32_t a0 = smem_u32(As), b0 = smem_u32(Bs);
+    };
+    auto any = [&](bool flag) { return __syncthreads_or(flag) != 0; };
+    auto issue = [&](int it, int s) {
+        if (tid != 0) return;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        const uint32_t a0 = smem_u32(tc_smem + s * SM::STAGE), b0 = a0 + SM::A;
 #pragma unroll
-            for (int q = 0; q < TC_BK / 16; ++q) {
-                const uint64_t da = tc_smem_desc(a0 + q * 256, 128, TC_SBO);
-                const uint64_t db = tc_smem_desc(b0 + q * 256, 128, TC_SBO);
-                const uint32_t acc = (it > 0 || q > 0) ? 1u : 0u;
-                asm volatile(
-                    "{\n\t.reg .pred p;\n\t"
-                    "setp.ne.b32 p, %4, 0;\n\t"
-                    "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-                    ::"r"(tmem), "l"(da), "l"(db), "r"(tc_idesc(TC_BM, TN)), "r"(acc)
-                    : "memory");
-            }
-            asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];"
-                         ::"r"(smem_u32(&mbar[s])) : "memory");
+        for (int q = 0; q < TC_BK / 16; ++q) {
+            const uint64_t da = tc_smem_desc(a0 + q * 256, 128, TC_SBO);
+            const uint64_t db = tc_smem_desc(b0 + q * 256, 128, TC_SBO);
+            const uint32_t acc = (it > 0 || q > 0) ? 1u : 0u;
+            asm volatile(
+                "{\n\t.reg .pred p;\n\t"
+                "setp.ne.b32 p, %4, 0;\n\t"
+                "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+                ::"r"(tmem), "l"(da), "l"(db), "r"(tc_idesc(TC_BM, TN)), "r"(acc)
+                : "memory");
         }
-    }
+        asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];"
+                     ::"r"(smem_u32(&mbar[s])) : "memory");
+    };
     // the last commit covers every MMA before it; after a wait that gave up it is the one bounded wait for what may
     // still be running before the tensor memory is released (the tile is then not written)
-    if (steps > 0) {
-        const int last = steps - 1;
-        if (!tc_wait(smem_u32(&mbar[last % TC_STAGES]), (uint32_t)((last / TC_STAGES) & 1))) atomicExch(&fail_sh, 1);
+    const bool ok = run_ring<TC_STAGES>(steps, wait, fill, any, issue);
+    if (tid == 0 && !ok) {
+        fail_sh = 1;   // for the cluster, which reads it after its barrier
+        atomicExch(&g_tc_status, 1);
     }
-    __syncthreads();
-    if (tid == 0 && fail_sh) atomicExch(&g_tc_status, 1);
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const int row = (warp & 3) * 32 + lane, c_begin = (warp >> 2) * (TN / 2);
     float* part = (float*)tc_smem;
-    if (split > 1 || fail_sh == 0) {
+    if (split > 1 || ok) {
 #pragma unroll 1
         for (int c0 = c_begin; c0 < c_begin + TN / 2; c0 += 16) {
             uint32_t r[16];
