@@ -392,8 +392,8 @@ __global__ void __launch_bounds__(TC_THREADS, 2) gemm_bf16_tc_kernel(const __gri
         asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];"
                      ::"r"(smem_u32(&mbar[s])) : "memory");
     };
-    // the last commit covers every MMA before it; after a wait that gave up it is the one bounded wait for what may
-    // still be running before the tensor memory is released (the tile is then not written)
+    // after a wait that gave up the tile is not written: its MMAs may be incomplete, and where the last wait gave up too,
+    // still read the stages that the partial tile would overwrite
     const bool ok = run_ring<TC_STAGES>(steps, wait, fill, any, issue);
     if (tid == 0 && !ok) {
         fail_sh = 1;   // for the cluster, which reads it after its barrier
@@ -402,7 +402,7 @@ __global__ void __launch_bounds__(TC_THREADS, 2) gemm_bf16_tc_kernel(const __gri
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const int row = (warp & 3) * 32 + lane, c_begin = (warp >> 2) * (TN / 2);
     float* part = (float*)tc_smem;
-    if (split > 1 || ok) {
+    if (ok) {
 #pragma unroll 1
         for (int c0 = c_begin; c0 < c_begin + TN / 2; c0 += 16) {
             uint32_t r[16];

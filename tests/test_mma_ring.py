@@ -125,3 +125,10 @@ def test_work_in_time(ring, steps):
 def test_threads_stay_together_after_a_late_wait(ring, steps, slow):
     same, ok, issued = ring(steps, slow, 400)[:3]   # longer than every wait
     assert (same, ok) == (1, 0) and issued <= steps
+
+
+@pytest.mark.parametrize("steps,slow", [(1, 0), (4, 0), (5, 1), (5, 2), (8, 2), (8, 4), (8, 7), (13, 5), (13, 12)])
+def test_late_work_has_ended_when_the_threads_return(ring, steps, slow):
+    """Work later than one wait (20-35 ms) but not than the second one."""
+    same, ok, issued, running, refilled = ring(steps, slow, 45)
+    assert same and issued >= slow + 1 and running == 0 and refilled == 0
