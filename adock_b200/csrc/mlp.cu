@@ -313,7 +313,10 @@ __device__ __forceinline__ void tc_epilogue(const GemmArgs& g, int m, int n, con
     }
 }
 
+// The .aligned instructions below (cluster barriers, tcgen05 allocation and loads) need all lanes of a warp together; after a
+// branch or loop that lanes leave apart a __syncwarp() makes that certain.
 __device__ __forceinline__ void cluster_sync() {
+    __syncwarp();
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
@@ -344,6 +347,7 @@ __global__ void __launch_bounds__(TC_THREADS, 2) gemm_bf16_tc_kernel(const __gri
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 0) {
+        __syncwarp();
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
                      ::"r"(smem_u32(&tmem_base_sh)), "r"(TN) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
@@ -406,6 +410,7 @@ __global__ void __launch_bounds__(TC_THREADS, 2) gemm_bf16_tc_kernel(const __gri
 #pragma unroll 1
         for (int c0 = c_begin; c0 < c_begin + TN / 2; c0 += 16) {
             uint32_t r[16];
+            __syncwarp();
             if (steps > 0) {
                 asm volatile(
                     "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
@@ -463,6 +468,7 @@ __global__ void __launch_bounds__(TC_THREADS, 2) gemm_bf16_tc_kernel(const __gri
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     if (warp == 0) {
+        __syncwarp();
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TN) : "memory");
     }
