@@ -1108,7 +1108,10 @@ __global__ void __launch_bounds__(128) eg_kernel(const __grid_constant__ SearchP
 // A CTA takes one conformer and SA_ROT (or fewer) of its rotations. A warp works on 32 / W rotations at a time, W lanes
 // striding over the translations of each, with W the power of two (8 to 32) that covers them: a probe-filtered lattice
 // holds from a handful of points in a packed pocket to thousands in an open box. (A CTA of 256 threads per rotation ran
-// with 8 of them busy on 8 points: 196,608 rotations 2,764 us, now 230 us.)
+// with 8 of them busy on 8 points: 196,608 rotations 2,764 us, now 230 us.) Where a CTA has fewer rotations than warps (few
+// ligands) and the lattice has more than 32 points, its warps share a rotation's translations, else a rotation has one warp.
+// An open lattice of 1,000 points, 3,072 rotations of a ligand of 24 atoms: 256 threads per rotation 200 us, one warp per
+// rotation on 384 CTAs 370 us, now 167 us; 64 ligands 16.8, 13.0 and 13.3 ms.
 // Bound by the latency of the map gathers (L2; a rotation's positions share few sectors), hence 48 warps per SM and
 // eight gathers in flight per lane. Positions round to grid points by adding 1.5 * 2^23 (round to nearest even, like the
 // float-to-int conversion it replaces, which runs at a quarter of the rate), and one of the two penalty terms per axis is
@@ -1116,16 +1119,24 @@ __global__ void __launch_bounds__(128) eg_kernel(const __grid_constant__ SearchP
 #define SA_WARPS 4
 #define SA_ROT 32
 
+// The launch's CTAs are sized for a lattice of many points. With few, a CTA's own start (a chain of dependent loads) is most
+// of its time, so every f-th CTA takes its successors' rotations too and those end at once. One ligand, 3,072 rotations on
+// 3,072 CTAs or folded: 8 points 38 or 25 us, 1,000 points 167 or 370 us.
+__device__ __forceinline__ int stage_a_fold(int nT, int fold) { return nT <= 16 ? fold : (nT <= 32 ? (fold + 1) / 2 : 1); }
+
 template <typename GT>
 __global__ void __launch_bounds__(32 * SA_WARPS) stage_a_kernel(const __grid_constant__ SearchParams P, const float* conf, int C,
-                                                                const float* quats, int Q, int q_chunk, const float* trans,
+                                                                const float* quats, int Q, int q_chunk, int fold, const float* trans,
                                                                 const int* ntrans, int NT_MAX, const int* lig_box,
                                                                 float cap, float* best_e, int* best_i) {
     extern __shared__ float4 smem4[];
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     const int chunks = (Q + q_chunk - 1) / q_chunk;
-    const int lc = (int)(blockIdx.x / chunks), q0 = (int)(blockIdx.x % chunks) * q_chunk;
-    const int q1 = min(q0 + q_chunk, Q), l = lc / C;
+    const int lc = (int)(blockIdx.x / chunks), l = lc / C, chunk = (int)(blockIdx.x % chunks);
+    const int box = lig_box ? lig_box[l] : l;   // translations per ligand, or per box shared by ligands
+    const int nT = ntrans[box], f = stage_a_fold(nT, fold);
+    if (chunk % f) return;   // its rotations belong to an earlier CTA
+    const int q0 = chunk * q_chunk, q1 = min(q0 + q_chunk * f, Q);
     const int4 inf = P.info[l];
     const int n_at = inf.x, ri = inf.w;
     const int nx = (int)P.dims[3 * ri], ny = (int)P.dims[3 * ri + 1], nz = (int)P.dims[3 * ri + 2];
@@ -1144,13 +1155,15 @@ __global__ void __launch_bounds__(32 * SA_WARPS) stage_a_kernel(const __grid_con
     wide = __syncthreads_or(wide);
     const float magic = 12582912.f;   // 1.5 * 2^23
     const unsigned bits = 0x4B400000u, sy = (unsigned)nz, sx = (unsigned)(ny * nz);
-    const int box = lig_box ? lig_box[l] : l;   // translations per ligand, or per box shared by ligands
-    const int nT = ntrans[box];
     const int W = nT <= 8 ? 8 : (nT <= 16 ? 16 : 32), groups = 32 / W, row = P.AM + 1;
     float4* X = smem4 + (size_t)wid * 4 * row;   // [32 / W][AM + 1] rotated conformer + slot offset
     const float* p = conf + (long long)lc * P.AM * 3;
     const float* Tb = trans + (long long)box * NT_MAX * 3;
-    for (int qb = q0 + wid * groups; qb < q1; qb += SA_WARPS * groups) {
+    // warps per rotation: with more than one, each team of warps takes exactly one rotation
+    const int team = nT > 32 ? max(1, SA_WARPS / (q1 - q0)) : 1, member = wid % team;
+    __shared__ float team_e[SA_WARPS];
+    __shared__ int team_i[SA_WARPS];
+    for (int qb = q0 + wid / team * groups; qb < q1; qb += SA_WARPS / team * groups) {
         for (int t = lane; t < groups * n_at; t += 32) {
             const int h = t / n_at, a = t - h * n_at, q = min(qb + h, q1 - 1);
             float qw = quats[4 * q], qx = quats[4 * q + 1], qy = quats[4 * q + 2], qz = quats[4 * q + 3];
@@ -1170,7 +1183,7 @@ __global__ void __launch_bounds__(32 * SA_WARPS) stage_a_kernel(const __grid_con
         const float4* Xq = X + h * row;
         float be = 3.4e38f;
         int bi = 0;
-        for (int ti = lane & (W - 1); ti < nT; ti += W) {
+        for (int ti = (lane & (W - 1)) + W * member; ti < nT; ti += W * team) {
             const float T0 = Tb[3 * ti], T1 = Tb[3 * ti + 1], T2 = Tb[3 * ti + 2];
             float e = 0.f;
 #pragma unroll 8
@@ -1202,11 +1215,30 @@ __global__ void __launch_bounds__(32 * SA_WARPS) stage_a_kernel(const __grid_con
             const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
             if (oe < be || (oe == be && oi < bi)) { be = oe; bi = oi; }
         }
-        if ((lane & (W - 1)) == 0 && qb + h < q1) {
+        if (team > 1) {
+            if (lane == 0) {
+                team_e[wid] = be;
+                team_i[wid] = bi;
+            }
+        } else if ((lane & (W - 1)) == 0 && qb + h < q1) {
             best_e[(long long)lc * Q + qb + h] = be;
             best_i[(long long)lc * Q + qb + h] = bi;
         }
         __syncwarp();
+    }
+    if (team > 1) {
+        __syncthreads();
+        if (lane == 0 && member == 0) {
+            const int q = q0 + wid / team;
+            float be = team_e[wid];
+            int bi = team_i[wid];
+            for (int w = wid + 1; w < wid + team; ++w)
+                if (team_e[w] < be || (team_e[w] == be && team_i[w] < bi)) { be = team_e[w]; bi = team_i[w]; }
+            if (q < q1) {
+                best_e[(long long)lc * Q + q] = be;
+                best_i[(long long)lc * Q + q] = bi;
+            }
+        }
     }
 }
 
@@ -1543,11 +1575,15 @@ int launch_stage_a(const SearchParams& P, long long blocks, const float* conf, i
     const size_t smem = (size_t)SA_WARPS * 4 * (P.AM + 1) * sizeof(float4);
     ADOCK_CUDA(cudaFuncSetAttribute(stage_a_kernel<GT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     const long long lc = blocks / Q;   // (ligand, conformer) pairs
-    // 32 rotations per CTA share the conformer; fewer where that leaves SMs without a CTA
-    int q_chunk = SA_ROT;
-    while (q_chunk > 8 && lc * ((Q + q_chunk - 1) / q_chunk) < 4LL * sm_count()) q_chunk /= 2;
-    stage_a_kernel<GT><<<(unsigned)(lc * ((Q + q_chunk - 1) / q_chunk)), 32 * SA_WARPS, smem, st>>>(
-        P, conf, C, quats, Q, q_chunk, trans, ntrans, nt_max, lig_box, cap, best_e, best_i);
+    // 32 rotations per CTA share the conformer; fewer where that leaves an SM less than the 12 CTAs (48 warps) that hide the
+    // gathers' latency. A packed pocket's few points are too little work for so many CTAs: see stage_a_fold.
+    auto ctas = [&](int q) { return lc * ((Q + q - 1) / q); };
+    int q_chunk = SA_ROT, q_packed = SA_ROT;
+    while (q_packed > 8 && ctas(q_packed) < 4LL * sm_count()) q_packed /= 2;
+    while (q_chunk > 1 && ctas(q_chunk) < 12LL * sm_count()) q_chunk /= 2;
+    const int fold = max(1, q_packed / q_chunk);
+    stage_a_kernel<GT><<<(unsigned)ctas(q_chunk), 32 * SA_WARPS, smem, st>>>(P, conf, C, quats, Q, q_chunk, fold, trans, ntrans,
+                                                                             nt_max, lig_box, cap, best_e, best_i);
     ADOCK_CUDA(cudaGetLastError());
     return ADOCK_OK;
 }
