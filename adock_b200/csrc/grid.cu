@@ -57,7 +57,7 @@ struct FitPrm {
     float cutoff, rep_off;
     float g1_off, g1_k, g2_off, g2_k, hyd_bad, hyd_inv, hb_bad, hb_inv;   // as VinaPrm
     int falling;
-    float ion_rmin, ion_cut, rep_cap;                          // ion_rmin = 1 / minimum distance, ion_cut = 1 / cutoff^2
+    float ion_rmin2, ion_cut, rep_cap;                         // ion_rmin2 = minimum distance^2, ion_cut = 1 / cutoff^2
     int n_lt, n_rt;
     float rad_lig[64];   // in order of radius
     int out_slot[64];    // output map (and W column) of each (radius-ordered) type
@@ -204,21 +204,27 @@ __device__ __forceinline__ float exp2_ftz(float x) {
 // exactly 0 (falling ramps, bad < good, are gated separately): no branch, so a thread's two points stay in flight.
 #define FAR_AWAY 1e4f
 
-// Distances of an atom at offsets (dx, dy, dz) from the thread's points; rinv ~ 1 / r (finite at r = 0), far: beyond the
-// cutoff. r = r2 * rinv with one Newton step, so it is as exact as sqrtf.
+// 1 / x to 1 ulp; subnormal x counts as 0
+__device__ __forceinline__ float rcp_ftz(float x) {
+    float y;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+
+// Distances of an atom at offsets (dx, dy, dz) from the thread's points; far: beyond the cutoff. r = r2 / sqrt(r2) with one
+// Newton step, so it is as exact as sqrtf.
 template <int PP>
 struct Distances {
-    float r[PP], rinv[PP];
+    float r[PP], r2[PP];
     bool far[PP];
     __device__ __forceinline__ Distances(float ax, const float (&x)[PP], float dy, float dz, float cut2) {
 #pragma unroll
         for (int h = 0; h < PP; ++h) {
             const float dx = ax - x[h];
-            const float r2 = __fmaf_rn(dz, dz, __fmaf_rn(dx, dx, __fmul_rn(dy, dy)));
-            far[h] = r2 >= cut2;
-            rinv[h] = rsqrt_ftz(fmaxf(r2, 1e-20f));
-            const float y = r2 * rinv[h];
-            r[h] = __fmaf_rn(__fmaf_rn(-y, y, r2), 0.5f * rinv[h], y);
+            r2[h] = __fmaf_rn(dz, dz, __fmaf_rn(dx, dx, __fmul_rn(dy, dy)));
+            far[h] = r2[h] >= cut2;
+            const float rinv = rsqrt_ftz(fmaxf(r2[h], 1e-20f)), y = r2[h] * rinv;
+            r[h] = __fmaf_rn(__fmaf_rn(-y, y, r2[h]), 0.5f * rinv, y);
         }
     }
 };
@@ -340,7 +346,7 @@ __global__ void __launch_bounds__(Tile<PP>::THREADS, PP == 2 ? 3 : 8) grid_vina_
 
 // Fitted maps. Bound by instruction issue: six multiply-adds per (atom, point, type) beside the basis per radius; the
 // weights come from shared memory, once for a thread's two points. One point per thread with every staged atom tested took
-// 732 us for 8,000 receptor atoms, 81^3 points and 8 types, this 436 us.
+// 732 us for 8,000 receptor atoms, 81^3 points and 8 types, this 452 us.
 // Packed FP32 pairs for the two points (fma.rn.f32x2) were slower in both kernels (287 and 432 us): the exponentials, minima
 // and ramps stay scalar, so the registers and moves of the pairs cost more than the issue slots they save.
 template <int PP>
@@ -404,8 +410,8 @@ __global__ void __launch_bounds__(Tile<PP>::THREADS, PP == 2 ? 3 : 6) grid_fit_k
                     for (int h = 0; h < PP; ++h) {
                         on[h] = D.far[h] ? 0.f : 1.f;
                         r[h] = D.far[h] ? FAR_AWAY : D.r[h] - ra;
-                        const float ri = fminf(D.rinv[h], P.ion_rmin);   // 1 / max(r, ion_rmin)
-                        ion[h] = on[h] * (ri * ri - P.ion_cut);
+                        // 1 / max(r, minimum)^2 straight from r^2: one rounding less than by way of r
+                        ion[h] = D.far[h] ? 0.f : rcp_ftz(fmaxf(D.r2[h], P.ion_rmin2)) - P.ion_cut;
                     }
 #pragma unroll
                     for (int q = 0; q < FIT_GROUP; ++q) {
@@ -601,7 +607,7 @@ static int grid_fit_launch(const float* rec_xyz, const int* rec_ext, int n_rec, 
     P.hyd_bad = prm[7]; P.hyd_inv = ramp_inv(prm[6], prm[7]);
     P.hb_bad = prm[9]; P.hb_inv = ramp_inv(prm[8], prm[9]);
     P.falling = !(P.hyd_inv > 0.f && P.hb_inv > 0.f);
-    P.ion_rmin = prm[10] > 0.f ? 1.f / prm[10] : INFINITY; P.ion_cut = 1.f / (prm[0] * prm[0]); P.rep_cap = prm[11];
+    P.ion_rmin2 = prm[10] > 0.f ? prm[10] * prm[10] : 0.f; P.ion_cut = 1.f / (prm[0] * prm[0]); P.rep_cap = prm[11];
     P.n_lt = n_lt; P.n_rt = n_rt;
     int order[64];
     order_by_radius(rad_lig, n_lt, order);
