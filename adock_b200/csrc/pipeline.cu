@@ -288,7 +288,7 @@ __global__ void __launch_bounds__(1024) select_starts_kernel(int CQ, int n2, int
     int* idx = (int*)(ssm + n2);
     const int l = blockIdx.x;
     for (int j = threadIdx.x; j < n2; j += blockDim.x) {
-        float v = 3.4e38f;
+        float v = INFINITY;   // padding sorts behind every total, infinite ones too (their index is lower)
         if (j < CQ) {
             v = best_e[(long long)l * CQ + j] + e_conf[(long long)l * C + j / Q];
             if (!(v == v)) v = 3.4e38f;
@@ -353,7 +353,7 @@ __global__ void __launch_bounds__(256) cluster_kernel(const int4* info, int P, i
     const int l = blockIdx.x;
     const int na = max(info[l].x, 1);
     for (int j = threadIdx.x; j < n2; j += blockDim.x) {
-        double v = 1.7e308;
+        double v = INFINITY;   // padding sorts behind every pose, infinite energies too (their index is lower)
         if (j < P) {
             v = e_total[(long long)l * P + j];
             if (!(v == v)) v = 1.7e308;
