@@ -28,7 +28,7 @@ def test_clusters_with_infinite_energies(P):
     X = (torch.arange(2 * P, dtype=torch.float32) * 10)[:, None, None].expand(2 * P, kp.AM, 3).contiguous()   # all apart
     reps, n = kp.cluster(e.reshape(-1).to(DEV), X.to(DEV), 2, P, 2.0, min(P, 32))
     for l in range(2):
-        key = np.where(np.isnan(e[l]), 1.7e308, e[l].numpy())
+        key = np.where(np.isnan(e[l].numpy()), 1.7e308, e[l].numpy())
         assert reps[l].tolist() == np.argsort(key, kind="stable")[:min(P, 32)].tolist() and int(n[l]) == min(P, 32)
 
 
