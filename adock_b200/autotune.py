@@ -6,9 +6,10 @@ resident 128-thread blocks per SM, i.e. 128, 80 or 64 registers). Which is faste
 into the regime of a running search (optimised starts + 8 MC steps), then times 8 and 32 MC steps under each
 variant and keeps the one with the least time per step between the two; results are cached per (device name, AM,
 KM, map dtype) for the life of the process and in ``$ADOCK_TUNE_CACHE`` (a JSON file) if set. The
-variants' order follows the kernel's code: on the 256-ligand batch the 128-register variant now takes 1.44 ms per step,
-the others 2.22 and 2.44 ms. The two run lengths take out a launch's fixed part (ramp-up and tail), which differs between
-variants and would decide the time of one short sample.
+variants' order follows the kernel's code: with the present one the 128-register variant is the fastest over ligands of
+12-110 heavy atoms, FP32 and FP16 maps, 32 to 16,384 chains (24 atoms, 8,192 chains: 0.81 ms per step, the others 1.10
+and 1.03 ms; 110 atoms, 4,096 chains: 11.8 ms, 18.3 and 19.2 ms). The two run lengths take out a launch's fixed part
+(ramp-up and tail), which differs between variants and would decide the time of one short sample.
 """
 from __future__ import annotations
 

@@ -79,9 +79,8 @@ __device__ __forceinline__ void quat_apply_rotvec(float* q, float rx, float ry, 
     q[0] = w * nn; q[1] = x * nn; q[2] = y * nn; q[3] = z * nn;
 }
 
-// exp(x) = 2^(x log2 e) and 1 / sqrt(x) as the single hardware instructions that flush denormals. The compiler's
-// __expf and rsqrtf add a rescaling for denormal operands or results (3-4 instructions each); a term below 1e-38 adds
-// nothing to energies of kcal/mol size, and the distances are clamped far above it.
+// exp(x) = 2^(x log2 e) and 1 / sqrt(x) as single PTX instructions that count subnormal operands and results as 0: a term
+// below 1e-38 adds nothing to energies of kcal/mol size, and the distances are clamped far above it.
 __device__ __forceinline__ float exp_ftz(float x) {
     float y;
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(__fmul_rn(x, 1.44269504f)));

@@ -1,9 +1,10 @@
 // Device code of the search kernels (sm_100a), included by the per-grid-dtype translation units
 // (search_f32.cu, search_f16.cu, search_bf16.cu) that instantiate the launchers, and by search.cu.
 //
-// Execution model: one warp owns one chain (pose). Lanes own heavy atoms a = lane + 32*i (i < APL, AM = 32*APL)
-// whose ligand-frame coordinates, grid slot and torsion bitmask stay in registers for the whole chain. Per-warp
-// shared memory holds world coordinates, forces, torsion axes, the BFGS inverse Hessian and the state vectors.
+// Execution model: one warp owns one chain (pose). Lanes own heavy atoms a = lane + 32*i (i < APL, AM = 32*APL),
+// whose ligand-frame coordinates, grid slot and torsion bitmask are read from the working layout (L1, L2) in each
+// evaluation. Per-warp shared memory holds world coordinates, radii, forces, torsion axes, the BFGS inverse Hessian and
+// the state vectors.
 // The Monte-Carlo kernel is persistent: warps pull chains from a device work counter (longest ligands first),
 // so uneven ligands do not leave SMs idle at the tail.
 #pragma once
@@ -150,7 +151,7 @@ struct WSLayout {
 // Per-chain context (registers).
 template <int APL>
 struct Chain {
-    int na, nt, np, nrounds;
+    int na, nt, nrounds;
     float rg;
     const int2* pairs;
     const char* grid;
@@ -170,7 +171,7 @@ template <int APL, typename GT>
 __device__ __forceinline__ void load_chain(Chain<APL>& c, const SearchParams& P, const TypeTables& tt, int l, float* ws,
                                            const WSLayout& L, int lane, const int* nb, int nbn) {
     const int4 inf = P.info[l];
-    c.na = inf.x; c.nt = inf.y; c.np = inf.z;
+    c.na = inf.x; c.nt = inf.y;
     c.nrounds = (inf.z + 31) >> 5;
     const int ri = inf.w;
     c.rg = P.rg[l];
@@ -1077,7 +1078,7 @@ __global__ void __launch_bounds__(128, MINB) mc_kernel(const __grid_constant__ S
 
 template <int APL, typename GT, bool EX>
 __global__ void __launch_bounds__(128) eg_kernel(const __grid_constant__ SearchParams P, const int* chain_lig, int n,
-                                                 const float* state, float* e_out, float* g_out, int exact,
+                                                 const float* state, float* e_out, float* g_out,
                                                  const __grid_constant__ TypeTables ttg) {
     extern __shared__ float4 smem4[];
     __shared__ TypeTables tt;
@@ -1552,7 +1553,7 @@ static int launch_eg_t(const SearchParams& P, const int* cl, int n, const float*
     long long blocks = (n + wpb - 1) / wpb;
     const long long cap = (long long)sm_count() * 16;
     if (blocks > cap) blocks = cap;
-    kern<<<(unsigned)blocks, 32 * wpb, smem, st>>>(P, cl, n, state, e, g, exact, tt);
+    kern<<<(unsigned)blocks, 32 * wpb, smem, st>>>(P, cl, n, state, e, g, tt);
     ADOCK_CUDA(cudaGetLastError());
     return ADOCK_OK;
 }

@@ -4,7 +4,7 @@ A small MLP proposes the MC move of each chain: x [320 features of the chain's c
 SiLU(256) -> 64 outputs = Gaussian means (columns 0..25) and log standard deviations (32..57) of the move
 (translation 3 A, rotation vector 3 rad, torsion deltas 20 rad). Weights are BF16 on the tensor cores with FP32
 accumulation; training keeps FP32 master weights and Adam moments. Every kernel is the library's own
-(adock_gemm_bf16, adock_mlp_nll, adock_silu_backward, adock_bias_grad, adock_adam).
+(adock_mlp_forward, adock_mlp_loss_grad, adock_adam).
 
 Training data come from the plain search itself (``collect``): the MC kernel logs, for each accepted move that
 lowered the chain's energy, the features of the pre-move state and the state; the target is the move from that

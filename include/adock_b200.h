@@ -114,7 +114,9 @@ typedef struct {
     int exact;
     const int* order;          /* dev [N] processing order (longest first) or NULL */
     int* queue;                /* dev, 1 int work counter, zeroed by the call on `stream` */
-    unsigned long long* evals; /* dev, 2 counters (accumulated): energy evaluations, atom evaluations; or NULL */
+    unsigned long long* evals; /* dev, 2 counters (accumulated): energy evaluations, atom evaluations; or NULL. A
+                                  line-search point evaluated once more for its gradient counts once; iterations that
+                                  would only repeat one another are not run and do not count */
     int variant;               /* launch variant (0 = default; 1-3 = 4, 6, 8 resident blocks per SM), autotuned */
     /* learned proposal (no reference counterpart): target states [N, prop_k, 32] from adock_prop_sample for the
      * launch's steps (NULL = plain MC); a learned step proposes its target state (torsions past 20 unchanged);
